@@ -7,52 +7,232 @@
 //   burning ship         src/frac_burning_ship.c:7-24
 //   generalized celtic   src/frac_generalized_celtic.c:7-24
 //   mandel-celtic hybrid src/frac_variant.c:5-24
-// Every operation is an explicit __dmul_rn / __dadd_rn / __dsub_rn /
-// __ddiv_rn, which the compiler never fuses, so the counts are bit-exact
-// whatever -fmad says.
+// Every value is the IEEE double the reference's operation gives, so the
+// counts are bit-exact whatever -fmad says.
 //
-// Work split (the GPU form of src/render_threads.c:360-393): instead of a
-// mutex-protected next_line counter advanced by whole rows, each warp pulls
-// an 8x4 pixel tile from a global atomic counter.  Square-ish tiles keep the
-// 32 lanes of a warp on neighbouring pixels, whose counts are close, which
-// limits divergence; dynamic pulling balances the very uneven rows.  When a
-// 4-row band completes, the warp that finished it raises a host-visible
-// band flag (the analogue of lines_rendered[] + lines_rendered_cond).
+// What bounds it: the FP64 pipe, one warp instruction per 16 (DFMA) to 19
+// (DADD, DMUL) cycles of an SM, where an integer instruction takes about
+// half a cycle.  So an iteration spends three FP64 instructions, all DFMA:
+// the three additions (a + b = fma(a, 1, b); 2 wre wim + c_im in one, the
+// doubling being exact), and forms its three products on the integer pipes,
+// bit for bit as the FP64 pipe would (mul_round); the escape test compares
+// 20-bit magnitudes and adds in double only near the bailout.  Measured
+// (960x540, 5.4e9 pixel-iterations): 168.6 ms with the nine FP64
+// instructions this replaces and whole tiles, 40.4 ms now; 122 warp
+// instructions an iteration, 65 SM cycles, the FP64 pipe 74% busy.
+//
+// An orbit whose (wre, wim) returns, bit for bit, to an earlier value repeats
+// for ever and never escapes: the pixel's count is 0 whatever the depth.  Each
+// iteration compares the state with the one kept at the last power of two
+// (Brent's cycle search); a pixel inside an attracting cycle's basin
+// converges to its cycle in a few hundred iterations.
+//
+// Work split (the GPU form of src/render_threads.c:360-393): warps pull 8x4
+// pixel tiles from a global atomic counter, in place of a mutex-protected
+// next_line counter advanced by whole rows, and a lane takes a new pixel as
+// soon as kRefill lanes are idle (pixel_feed.cuh).
 #include "internal.h"
+#include "pixel_feed.cuh"
 
 namespace mdz {
 namespace {
 
-constexpr int kTileW = 8;
-constexpr int kTileH = 4;
-constexpr int kBlock = 256;
+constexpr int kBlock = 128;
+constexpr int kRefill = 3;        // idle lanes that make a warp take new pixels
+constexpr int kRefillEvery = 4;   // iterations between looks at the idle lanes
+// 16 warps an SM keep the FP64 pipe as busy as 32 do and take twice the tiles
+// each, so fewer lanes idle at the frame's end (960x540 to depth 20000 around
+// a boundary point: 40.4 ms with 16 warps, 42.4 with 24, 46.6 with 32, 46.7
+// with 10; refill at 3 idle lanes 40.4 ms, at 6 42.0 ms).
+constexpr int kBlocksPerSm = 4;
 
-template <int FRACTAL, bool JULIA>
-__device__ __forceinline__ uint32_t escape_fp64(double x, double y, double jre,
-                                                double jim, uint32_t depth)
+// a b + c, never simplified to an addition or a product
+__device__ __forceinline__ double dfma(double a, double b, double c)
 {
-    double wre = x, wim = y;
-    double wre2 = __dmul_rn(x, x);
-    double wim2 = __dmul_rn(y, y);
-    const double c_re = JULIA ? jre : x;
-    const double c_im = JULIA ? jim : y;
-    for (uint32_t wz = 1; wz <= depth; ++wz) {
-        double t;
-        if (FRACTAL == MDZ_BURNING_SHIP)
-            t = __dmul_rn(2.0, fabs(__dmul_rn(wre, wim)));  // 2.0 * fabsl(wre * wim)
-        else
-            t = __dmul_rn(__dmul_rn(2.0, wre), wim);         // 2.0 * wre * wim
-        wim = __dadd_rn(t, c_im);
-        double d = __dsub_rn(wre2, wim2);
-        if (FRACTAL == MDZ_GENERALIZED_CELTIC || (FRACTAL == MDZ_VARIANT && (wz & 1u)))
-            d = fabs(d);
-        wre = __dadd_rn(d, c_re);
-        wim2 = __dmul_rn(wim, wim);
-        wre2 = __dmul_rn(wre, wre);
-        if (__dadd_rn(wim2, wre2) > 4.0)
-            return wz;
+    double r;
+    asm("fma.rn.f64 %0, %1, %2, %3;" : "=d"(r) : "d"(a), "d"(b), "d"(c));
+    return r;
+}
+
+// A double cut in three: its mantissa with the leading 1 (h: top 21 bits,
+// l: low 32) and q = high word - h, its sign and exponent field less one.
+struct Split {
+    uint32_t h, l, q;
+};
+
+__device__ __forceinline__ Split split(double x)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(x);
+    const uint32_t h = (hi & 0x000fffffu) | 0x00100000u;
+    return Split{h, (uint32_t)__double2loint(x), hi - h};
+}
+
+// Whether one of the two has an exponent outside 2^-479 .. 2^32 (0,
+// denormals, infinities and NaN are outside): inside, no product of the two
+// leaves the normal range, and its magnitude fits a float's exponent.  The
+// sign bit falls out of the mask.
+__device__ __forceinline__ bool odd_exponent(const Split& x, const Split& y)
+{
+    const uint32_t lowest = 0x22000000u - 0x00100000u;
+    return (((x.q - lowest) | (y.q - lowest)) & 0x60000000u) != 0u;
+}
+
+// x y rounded to nearest from the product of the mantissas, H 2^64 + m 2^32 +
+// t (t's low word is not needed); q is the sum of the operands' q.  Returns
+// true when the bits below the result's last place are 100..0 as far as m
+// goes: t or the parity decides there, and the caller multiplies in double.
+__device__ __forceinline__ bool round106(uint64_t H, uint64_t m, uint64_t t, uint32_t q,
+                                         uint32_t& hi, uint32_t& lo)
+{
+    uint32_t v, hl, hh;   // bits 32.., 64.., 96.. of the product
+    asm("{add.cc.u32 %0, %3, %4;\n\t"
+        "addc.cc.u32 %1, %5, %6;\n\t"
+        "addc.u32 %2, %7, 0;}"
+        : "=&r"(v), "=&r"(hl), "=r"(hh)
+        : "r"((uint32_t)m), "r"((uint32_t)(t >> 32)), "r"((uint32_t)H), "r"((uint32_t)(m >> 32)),
+          "r"((uint32_t)(H >> 32)));
+    const uint32_t s = hh >> 9;          // 1: the mantissas' product is 2 or more
+    const uint32_t sh = 12u - s;
+    const uint32_t r = v << sh;          // what is rounded away
+    asm("{.reg .u32 c;\n\t"
+        "add.cc.u32 c, %2, %2;\n\t"      // carry = r >> 31: round up
+        "addc.cc.u32 %0, %3, 0;\n\t"
+        "addc.u32 %1, %4, %5;}"
+        : "=&r"(lo), "=r"(hi)
+        : "r"(r), "r"(__funnelshift_l(v, hl, sh)), "r"(__funnelshift_l(hl, hh, sh)),
+          "r"(q + (s << 20) + (0x00200000u - 0x40000000u)));
+    return r == 0x80000000u;
+}
+
+__device__ __forceinline__ uint64_t wide(uint32_t a, uint32_t b)
+{
+    return (uint64_t)a * b;
+}
+
+__device__ __forceinline__ bool mul_round(const Split& x, const Split& y, uint32_t& hi,
+                                          uint32_t& lo)
+{
+    return round106(wide(x.h, y.h), wide(x.h, y.l) + wide(y.h, x.l), wide(x.l, y.l), x.q + y.q, hi,
+                    lo);
+}
+
+__device__ __forceinline__ bool sqr_round(const Split& x, uint32_t& hi, uint32_t& lo)
+{
+    return round106(wide(x.h, x.h), wide(2u * x.h, x.l), wide(x.l, x.l), 2u * x.q, hi, lo);
+}
+
+// A double's high word as a float cut to 20 bits: right for 2^-126 .. 2^128;
+// of a smaller or larger one only the bits' sign and pattern are left.
+__device__ __forceinline__ float cut20(double x)
+{
+    return __int_as_float((int)((uint32_t)__double2hiint(x) * 8u - 0xc0000000u));
+}
+
+// One pixel's orbit between iterations.
+struct Orbit {
+    double wre, wim, wre2, wim2;
+    double c_re, c_im;
+    double kre, kim;      // state kept for the cycle search
+    Split r, i;           // of wre, wim
+    uint32_t wz;          // iterations done
+    uint32_t event;       // iteration after which the state is kept, or depth
+    bool odd;             // a component's exponent is odd: next product in double
+};
+
+__device__ __forceinline__ void orbit_start(Orbit& o, double x, double y, double c_re, double c_im,
+                                            uint32_t depth)
+{
+    o.wre = o.kre = x;
+    o.wim = o.kim = y;
+    o.c_re = c_re;
+    o.c_im = c_im;
+    o.wz = 0;
+    o.event = min(2u, depth);
+    o.r = split(x);
+    o.i = split(y);
+    o.odd = odd_exponent(o.r, o.i);
+    o.wre2 = __dmul_rn(x, x);
+    o.wim2 = __dmul_rn(y, y);
+}
+
+// The iteration as the reference writes it, in double throughout: z and its
+// squares after iteration o.wz from (re, im, re2, im2).
+template <int FRACTAL>
+__device__ __forceinline__ void orbit_step_double(Orbit& o, double re, double im, double re2,
+                                                  double im2)
+{
+    const double t = FRACTAL == MDZ_BURNING_SHIP ? __dmul_rn(2.0, fabs(__dmul_rn(re, im)))
+                                                 : __dmul_rn(__dmul_rn(2.0, re), im);
+    double d = __dsub_rn(re2, im2);
+    if (FRACTAL == MDZ_GENERALIZED_CELTIC || (FRACTAL == MDZ_VARIANT && (o.wz & 1u)))
+        d = fabs(d);
+    o.wim = __dadd_rn(t, o.c_im);
+    o.wre = __dadd_rn(d, o.c_re);
+    o.r = split(o.wre);
+    o.i = split(o.wim);
+    o.odd = odd_exponent(o.r, o.i);
+    o.wim2 = __dmul_rn(o.wim, o.wim);
+    o.wre2 = __dmul_rn(o.wre, o.wre);
+}
+
+// The next iteration.  Returns true when the pixel is done, with its count.
+template <int FRACTAL>
+__device__ __forceinline__ bool orbit_step(Orbit& o, uint32_t depth, double one, double two,
+                                           uint32_t& count)
+{
+    uint32_t hi, lo;
+    const double re = o.wre, im = o.wim, re2 = o.wre2, im2 = o.wim2;
+    ++o.wz;
+    bool hard = mul_round(o.r, o.i, hi, lo) | o.odd;
+    if (FRACTAL == MDZ_BURNING_SHIP)
+        hi &= 0x7fffffffu;
+    // 2.0 * wre * wim + c_im, burning ship 2.0 * fabsl(wre * wim) + c_im
+    o.wim = dfma(__hiloint2double((int)hi, (int)lo), two, o.c_im);
+    double d = dfma(im2, -one, re2);
+    if (FRACTAL == MDZ_GENERALIZED_CELTIC || (FRACTAL == MDZ_VARIANT && (o.wz & 1u)))
+        d = __hiloint2double(__double2hiint(d) & 0x7fffffff, __double2loint(d));
+    o.wre = dfma(d, one, o.c_re);
+    o.r = split(o.wre);
+    o.i = split(o.wim);
+    o.odd = odd_exponent(o.r, o.i);
+    hard |= sqr_round(o.i, hi, lo) | o.odd;
+    o.wim2 = __hiloint2double((int)hi, (int)lo);
+    hard |= sqr_round(o.r, hi, lo);
+    o.wre2 = __hiloint2double((int)hi, (int)lo);
+    if (hard)   // one lane in ~10^6, and zeros
+        orbit_step_double<FRACTAL>(o, re, im, re2, im2);
+    // |z|^2 > 4: a cut is below its value by at most 2^-20 of it; of a value
+    // below 2^-126 it is some positive number or NaN, which hides no escape
+    if (!(fabsf(cut20(o.wim2)) + fabsf(cut20(o.wre2)) <= 3.9999f) || hard) {
+        double m;   // volatile: computed here only
+        asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(m) : "d"(o.wim2), "d"(o.wre2));
+        if (m > 4.0) {
+            count = o.wz;
+            return true;
+        }
     }
-    return 0;
+    // the states kept are the start's and those after iterations 2, 4, 8, ..,
+    // so the hybrid's formula agrees too when wz is even
+    if (((__double2loint(o.wre) ^ __double2loint(o.kre))
+         | (__double2loint(o.wim) ^ __double2loint(o.kim)))
+        == 0) {
+        if (__double2hiint(o.wre) == __double2hiint(o.kre)
+            && __double2hiint(o.wim) == __double2hiint(o.kim)
+            && (FRACTAL != MDZ_VARIANT || (o.wz & 1u) == 0u)) {
+            count = 0;
+            return true;
+        }
+    }
+    if (o.wz == o.event) {
+        if (o.wz >= depth) {
+            count = 0;
+            return true;
+        }
+        o.kre = o.wre;
+        o.kim = o.wim;
+        o.event = min(o.event * 2u, depth);
+    }
+    return false;
 }
 
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
@@ -66,49 +246,80 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 template <int FRACTAL, bool JULIA>
 __global__ void __launch_bounds__(kBlock) fp64_frame_kernel(Fp64Launch p)
 {
-    const int lane = threadIdx.x & 31;
+    // the warp's current tile
+    struct Pixel {
+        double x, y;
+        int ix, row;
+    };
+    __shared__ Pixel tile[kBlock / 32][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tiles_x = (p.W + kTileW - 1) / kTileW;
     const int tiles_y = (p.nrows + kTileH - 1) / kTileH;
     const unsigned total = (unsigned)tiles_x * (unsigned)tiles_y;
     const double width = __dsub_rn(p.xmax, p.xmin);
     const double fw = (double)p.W;
     const double ystep = __ddiv_rn(width, fw);
+    unsigned long long its = 0;
+    TileFeed feed;
+    bool active = false;           // this lane iterates a pixel
+    int ix = 0, lrow = 0;
+    int band = -1;
+    Orbit o;
     for (;;) {
-        unsigned t = 0;
-        if (lane == 0)
-            t = (p.stop && *p.stop) ? total : atomicAdd(&p.sync->tile_counter, 1u);
-        t = __shfl_sync(0xffffffffu, t, 0);
-        if (t >= total)
+        if (p.tile_rows_done)
+            count_bands(p.W, p.nrows, p.tile_rows_done, p.band_flags, band);
+        feed_lanes(
+            feed, !active,
+            [&]() {
+                unsigned t = 0;
+                if (lane == 0)
+                    t = (p.stop && *p.stop) ? total : atomicAdd(&p.sync->tile_counter, 1u);
+                t = __shfl_sync(0xffffffffu, t, 0);
+                return t < total ? t : ~0u;
+            },
+            [&](unsigned t, int& px, int& row) {
+                const int ty = (int)(t / (unsigned)tiles_x);
+                px = (int)(t - (unsigned)ty * (unsigned)tiles_x) * kTileW + (lane & (kTileW - 1));
+                row = ty * kTileH + lane / kTileW;
+                return px < p.W && row < p.nrows;
+            },
+            [&](int k, int px, int row) {
+                const double y = __dsub_rn(p.ymax, __dmul_rn(ystep, (double)(p.row0 + row)));
+                const double x = __dadd_rn(__dmul_rn(__ddiv_rn((double)px, fw), width), p.xmin);
+                tile[warp][k] = Pixel{x, y, px, row};
+            },
+            [&](int k) {
+                const Pixel& q = tile[warp][k];
+                ix = q.ix;
+                lrow = q.row;
+                orbit_start(o, q.x, q.y, JULIA ? p.jre : q.x, JULIA ? p.jim : q.y, p.depth);
+                active = true;
+            });
+        if (!__any_sync(0xffffffffu, active))
             break;
-        const int ty = (int)(t / (unsigned)tiles_x);
-        const int tx = (int)(t - (unsigned)ty * (unsigned)tiles_x);
-        const int ix = tx * kTileW + (lane & (kTileW - 1));
-        const int lrow = ty * kTileH + (lane / kTileW);
-        unsigned long long its = 0;
-        if (ix < p.W && lrow < p.nrows) {
-            const int line = p.row0 + lrow;
-            const double y = __dsub_rn(p.ymax, __dmul_rn(ystep, (double)line));
-            const double x =
-                __dadd_rn(__dmul_rn(__ddiv_rn((double)ix, fw), width), p.xmin);
-            const uint32_t n = escape_fp64<FRACTAL, JULIA>(x, y, p.jre, p.jim, p.depth);
-            p.out[(size_t)lrow * p.W + ix] = (int32_t)n;
-            its = n ? n : p.depth;
-        }
-        its = warp_sum_u64(its);
-        if (p.band_flags)
-            __threadfence_system();
-        __syncwarp();
-        if (lane == 0) {
-            atomicAdd(&p.sync->iter_sum, its);
-            if (p.tile_rows_done) {
-                const unsigned done = atomicAdd(&p.tile_rows_done[ty], 1u) + 1u;
-                if (done == (unsigned)tiles_x && p.band_flags) {
-                    __threadfence_system();
-                    p.band_flags[ty] = 1;
+        // iterate until enough lanes are idle to be worth a look
+        const int enough = (feed.left || feed.more) ? kRefill : 32;
+        do {
+            if (active) {
+                uint32_t n;
+                int u = kRefillEvery;
+                bool done;
+#pragma unroll 1
+                do
+                    done = orbit_step<FRACTAL>(o, p.depth, p.one, p.two, n);
+                while (!done && --u);
+                if (done) {
+                    p.out[(size_t)lrow * p.W + ix] = (int32_t)n;
+                    its += n ? n : p.depth;
+                    active = false;
+                    band = lrow / kTileH;
                 }
             }
-        }
+        } while (__popc(__ballot_sync(0xffffffffu, !active)) < enough);
     }
+    its = warp_sum_u64(its);
+    if (lane == 0 && its)
+        atomicAdd(&p.sync->iter_sum, its);
 }
 
 template <int FRACTAL, bool JULIA>
@@ -122,7 +333,7 @@ int launch_one(mdzgpu_ctx* ctx, const Fp64Launch& p, cudaStream_t s)
             blocks_per_sm = 1;
     }
     const long tiles = (long)((p.W + kTileW - 1) / kTileW) * ((p.nrows + kTileH - 1) / kTileH);
-    long grid = (long)ctx->num_sms * blocks_per_sm;
+    long grid = (long)ctx->num_sms * (blocks_per_sm < kBlocksPerSm ? blocks_per_sm : kBlocksPerSm);
     const long warps_needed = tiles;
     const long blocks_needed = (warps_needed + kBlock / 32 - 1) / (kBlock / 32);
     if (grid > blocks_needed)

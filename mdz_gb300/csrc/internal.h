@@ -121,9 +121,12 @@ struct Fp64Launch {
     double xmin, xmax, ymax, jre, jim;
     int32_t* out;       // out[(line - row0) * W + ix]
     FrameSync* sync;
-    unsigned int* tile_rows_done;  // per 4-row band
+    unsigned int* tile_rows_done;  // pixels done per 4-row band
     volatile int* band_flags;      // host-mapped, per 4-row band (may be null)
     volatile int* stop;            // host-mapped stop word (may be null)
+    // operands of the DFMAs that stand for additions, read from the launch's
+    // parameters so that the compiler keeps them DFMAs
+    double one = 1.0, two = 2.0;
 };
 int launch_fp64(mdzgpu_ctx* ctx, const Fp64Launch& p, cudaStream_t s);
 
