@@ -14,29 +14,38 @@
 // One thread iterates one pixel; magnitudes and sign masks are kept
 // separately so the three products per iteration run on magnitudes.  c stays
 // in registers up to 16 words and moves to shared memory above that so the
-// 34/36-word (1088-bit class) kernels fit in registers.  Work is pulled in
-// 8x4 tiles per warp from an atomic counter, as in the FP64 kernel.
+// 34/36-word (1088-bit class) kernels fit in registers.  Warps pull 8x4 tiles
+// (or 32 entries of a list) from an atomic counter, and a lane takes a new
+// pixel once kRefill lanes are idle (pixel_feed.cuh).
+//
+// What bounds it is the integer multiplier: N = 10 takes 126 partial products
+// an iteration at 1.1 cycles of an SM each, N = 34 1272 (fixed_point.cuh).
+#include <type_traits>
+
 #include "fixed_point.cuh"
 #include "internal.h"
+#include "pixel_feed.cuh"
 #include "serve.h"
 
 namespace mdz {
 namespace {
 
-constexpr int kTileW = 8;
-constexpr int kTileH = 4;
+constexpr int kRefill = 4;        // idle lanes that make a warp take new pixels
+constexpr int kRefillEvery = 8;   // iterations between looks at the idle lanes
 
 template <int N>
 struct CRegs {
     uint32_t w[N];
     __device__ __forceinline__ uint32_t operator()(int k) const { return w[k]; }
+    __device__ __forceinline__ void set(int k, uint32_t v) { w[k] = v; }
 };
 
 template <int N>
 struct CShared {
-    const uint32_t* base;  // word k of this thread at base[k * stride]
+    uint32_t* base;  // word k of this thread at base[k * stride]
     int stride;
     __device__ __forceinline__ uint32_t operator()(int k) const { return base[k * stride]; }
+    __device__ __forceinline__ void set(int k, uint32_t v) { base[k * stride] = v; }
 };
 
 // Top two words of a fixed-point number as a float (value < 128 in size).
@@ -47,106 +56,69 @@ __device__ __forceinline__ float fx_top_float(const uint32_t (&x)[N])
            + (float)x[N - 2] * 1.3877788e-17f /* 2^-56 */;
 }
 
-template <int N, int FRACTAL, class CG>
-__device__ __forceinline__ uint32_t escape_mp(uint32_t (&wre)[N], uint32_t (&wim)[N],
-                                              const CG& c_re, const CG& c_im, uint32_t depth,
-                                              float& mag)
+// A pixel's orbit between iterations: |wre|, |wim| with their sign masks and
+// wre^2 - wim^2, after `wz` iterations.
+template <int N>
+struct MpOrbit {
+    uint32_t wre[N], wim[N], d[N];
+    uint32_t sre, sim;
+    uint32_t wz;
+};
+
+// The squares of |wre|, |wim|: sets d; returns whether |z|^2 > 4, and |z|^2
+// (rounded) when it is or when `want_mag`.
+template <int N>
+__device__ __forceinline__ bool mp_squares(MpOrbit<N>& o, bool want_mag, float& mag)
 {
-    uint32_t wre2[N], wim2[N], acc[N + 2], t[N], d[N];
-    uint32_t sre = fx::abs_inplace<N>(wre);
-    uint32_t sim = fx::abs_inplace<N>(wim);
-    fx::sqr_trunc<N>(wre, acc);
-    fx::extract<N, 24>(acc, wre2);
-    fx::sqr_trunc<N>(wim, acc);
+    uint32_t acc[N + 2], wre2[N], wim2[N];
+    fx::sqr_trunc<N>(o.wim, acc);
     fx::extract<N, 24>(acc, wim2);
-    for (uint32_t wz = 1; wz <= depth; ++wz) {
-        // wim = 2.0 * wre * wim + c_im   (burning ship: 2 |wre wim| + c_im)
-        fx::mul_trunc<N>(wre, wim, acc);
-        fx::extract<N, 23>(acc, t);
-        const uint32_t mt = (FRACTAL == MDZ_BURNING_SHIP) ? 0u : (sre ^ sim);
-        fx::add_signed<N>(c_im, t, mt, wim);
-        // wre = wre2 - wim2 + c_re       (celtic: |wre2 - wim2| + c_re)
-        fx::sub<N>(wre2, wim2, d);
-        uint32_t md = 0u;
-        if (FRACTAL == MDZ_GENERALIZED_CELTIC || (FRACTAL == MDZ_VARIANT && (wz & 1u)))
-            md = (uint32_t)((int32_t)d[N - 1] >> 31);
-        fx::add_signed<N>(c_re, d, md, wre);
-        if (fx::big<N>(wre) || fx::big<N>(wim)) {
-            const float a = fx_top_float<N>(wre), b = fx_top_float<N>(wim);
-            mag = a * a + b * b;
-            return wz;
-        }
-        sre = fx::abs_inplace<N>(wre);
-        sim = fx::abs_inplace<N>(wim);
-        // wim2 = wim * wim; wre2 = wre * wre
-        fx::sqr_trunc<N>(wim, acc);
-        fx::extract<N, 24>(acc, wim2);
-        fx::sqr_trunc<N>(wre, acc);
-        fx::extract<N, 24>(acc, wre2);
-        if (fx::sum_gt4<N>(wim2, wre2)) {
-            mag = fx_top_float<N>(wim2) + fx_top_float<N>(wre2);
-            return wz;
-        }
-    }
-    mag = fx_top_float<N>(wim2) + fx_top_float<N>(wre2);
-    return 0;
+    fx::sqr_trunc<N>(o.wre, acc);
+    fx::extract<N, 24>(acc, wre2);
+    const bool escaped = fx::sum_gt4<N>(wim2, wre2);
+    if (escaped || want_mag)
+        mag = fx_top_float<N>(wim2) + fx_top_float<N>(wre2);
+    fx::sub<N>(wre2, wim2, o.d);
+    return escaped;
 }
 
-// Resumable form for the serving engine: enters with |wre|, |wim| and their
-// sign masks after iteration wz - 1, runs iterations wz .. last (<= depth)
-// with the formula chosen at run time, and returns true when the pixel is
-// finished (count in wz: the escape iteration, or 0 at depth); false leaves
-// the state after iteration `last` (wz = last + 1).  The operations are
-// those of escape_mp, so a pixel split over any number of calls gets the
-// same count.
-template <int N, class CG>
-__device__ __forceinline__ bool escape_mp_resume(uint32_t (&wre)[N], uint32_t (&wim)[N],
-                                                 uint32_t& sre, uint32_t& sim, const CG& c_re,
-                                                 const CG& c_im, int fractal, uint32_t& wz,
-                                                 uint32_t last, uint32_t depth, float& mag)
+// Signs and magnitudes of a start value in wre, wim.
+template <int N>
+__device__ __forceinline__ void mp_start(MpOrbit<N>& o)
 {
-    uint32_t wre2[N], wim2[N], acc[N + 2], t[N], d[N];
-    fx::sqr_trunc<N>(wre, acc);
-    fx::extract<N, 24>(acc, wre2);
-    fx::sqr_trunc<N>(wim, acc);
-    fx::extract<N, 24>(acc, wim2);
-    const bool ship = fractal == MDZ_BURNING_SHIP;
-    const bool celtic = fractal == MDZ_GENERALIZED_CELTIC;
-    const bool variant = fractal == MDZ_VARIANT;
-    if (last > depth)
-        last = depth;
-    for (; wz <= last; ++wz) {
-        fx::mul_trunc<N>(wre, wim, acc);
-        fx::extract<N, 23>(acc, t);
-        const uint32_t mt = ship ? 0u : (sre ^ sim);
-        fx::add_signed<N>(c_im, t, mt, wim);
-        fx::sub<N>(wre2, wim2, d);
-        uint32_t md = 0u;
-        if (celtic || (variant && (wz & 1u)))
-            md = (uint32_t)((int32_t)d[N - 1] >> 31);
-        fx::add_signed<N>(c_re, d, md, wre);
-        if (fx::big<N>(wre) || fx::big<N>(wim)) {
-            const float a = fx_top_float<N>(wre), b = fx_top_float<N>(wim);
-            mag = a * a + b * b;
-            return true;
-        }
-        sre = fx::abs_inplace<N>(wre);
-        sim = fx::abs_inplace<N>(wim);
-        fx::sqr_trunc<N>(wim, acc);
-        fx::extract<N, 24>(acc, wim2);
-        fx::sqr_trunc<N>(wre, acc);
-        fx::extract<N, 24>(acc, wre2);
-        if (fx::sum_gt4<N>(wim2, wre2)) {
-            mag = fx_top_float<N>(wim2) + fx_top_float<N>(wre2);
-            return true;
-        }
-    }
-    mag = fx_top_float<N>(wim2) + fx_top_float<N>(wre2);
-    if (wz > depth) {
-        wz = 0;
+    float mag;
+    o.sre = fx::abs_inplace<N>(o.wre);
+    o.sim = fx::abs_inplace<N>(o.wim);
+    o.wz = 0;
+    mp_squares<N>(o, false, mag);   // z_0 = c is not tested
+}
+
+// The next iteration.  Returns true when z escaped; mag as mp_squares.
+// `fold_im`: burning ship; `fold_re`: celtic; `fold_odd`: the hybrid's fold
+// on odd iterations.
+template <int N, class CG>
+__device__ __forceinline__ bool mp_step(MpOrbit<N>& o, const CG& c_re, const CG& c_im, bool fold_im,
+                                        bool fold_re, bool fold_odd, bool want_mag, float& mag)
+{
+    uint32_t acc[N + 2], t[N];
+    ++o.wz;
+    // wim = 2.0 * wre * wim + c_im   (burning ship: 2 |wre wim| + c_im)
+    fx::mul_trunc<N>(o.wre, o.wim, acc);
+    fx::extract<N, 23>(acc, t);
+    fx::add_signed<N>(c_im, t, fold_im ? 0u : (o.sre ^ o.sim), o.wim);
+    // wre = wre2 - wim2 + c_re       (celtic: |wre2 - wim2| + c_re)
+    const uint32_t md = (fold_re || (fold_odd && (o.wz & 1u)))
+                            ? (uint32_t)((int32_t)o.d[N - 1] >> 31)
+                            : 0u;
+    fx::add_signed<N>(c_re, o.d, md, o.wre);
+    if (fx::big<N>(o.wre) || fx::big<N>(o.wim)) {
+        const float a = fx_top_float<N>(o.wre), b = fx_top_float<N>(o.wim);
+        mag = a * a + b * b;
         return true;
     }
-    return false;
+    o.sre = fx::abs_inplace<N>(o.wre);
+    o.sim = fx::abs_inplace<N>(o.wim);
+    return mp_squares<N>(o, want_mag, mag);
 }
 
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
@@ -163,98 +135,128 @@ __host__ __device__ constexpr bool c_in_smem()
     return N > 16;
 }
 
+// Threads of a serving block.
 template <int N>
 __host__ __device__ constexpr int block_threads()
 {
     return N > 16 ? 128 : 256;
 }
 
+// Frame launches take blocks of four warps, one for each of an SM's schedulers,
+// so that a frame or list of few tiles spreads over all SMs (blocks of eight
+// left the 949 tiles of a 201x151 frame at N = 34 70 to 86 ms, against 66),
+// and at most 16 warps an SM: with 24 nothing gains (640x480-class frames at
+// 4 and 10 words, within 3%), with 8 the multiplier waits (27 -> 29 ms).
+constexpr int kFrameBlock = 128;
+
+template <int N>
+__host__ __device__ constexpr int frame_blocks_per_sm()
+{
+    return N > 20 ? 2 : N > 16 ? 3 : 4;
+}
+
 template <int N, int FRACTAL, bool JULIA>
-__global__ void __launch_bounds__(block_threads<N>()) mp_frame_kernel(MpLaunch p)
+__global__ void __launch_bounds__(kFrameBlock, frame_blocks_per_sm<N>())
+    mp_frame_kernel(MpLaunch p)
 {
     extern __shared__ uint32_t smem[];
-    const int lane = threadIdx.x & 31;
+    __shared__ int2 tile[kFrameBlock / 32][32];   // the warp's current tile
+    using CGet = typename std::conditional<c_in_smem<N>(), CShared<N>, CRegs<N>>::type;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tiles_x = (p.W + kTileW - 1) / kTileW;
     const int tiles_y = (p.nrows + kTileH - 1) / kTileH;
     const unsigned list_n = p.list ? *p.list_count : 0u;
     const unsigned total = p.list ? (list_n + 31u) / 32u : (unsigned)tiles_x * (unsigned)tiles_y;
+    unsigned long long its = 0;
+    TileFeed feed;
+    bool active = false;   // this lane iterates a pixel
+    int ix = 0, lrow = 0;
+    int band = -1;
+    MpOrbit<N> o;
+    CGet c_re, c_im;
+    if constexpr (c_in_smem<N>()) {
+        c_re = CGet{smem + threadIdx.x, kFrameBlock};
+        c_im = CGet{smem + N * kFrameBlock + threadIdx.x, kFrameBlock};
+    }
     for (;;) {
-        unsigned tile = 0;
-        if (lane == 0) {
-            const unsigned t = (p.stop && *p.stop) ? 0xffffffffu
-                                                    : atomicAdd(&p.sync->tile_counter, 1u);
-            tile = t >= p.tile_limit ? total : p.tile_base + t;
-        }
-        tile = __shfl_sync(0xffffffffu, tile, 0);
-        if (tile >= total)
-            break;
-        int ix, lrow, ty = 0;
-        bool valid;
-        if (p.list) {
-            const unsigned i = tile * 32u + lane;
-            valid = i < list_n;
-            const unsigned pix = valid ? p.list[i] : 0u;
-            lrow = (int)(pix / (unsigned)p.W);
-            ix = (int)(pix - (unsigned)lrow * (unsigned)p.W);
-        } else {
-            ty = (int)(tile / (unsigned)tiles_x);
-            const int tx = (int)(tile - (unsigned)ty * (unsigned)tiles_x);
-            ix = tx * kTileW + (lane & (kTileW - 1));
-            lrow = ty * kTileH + (lane / kTileW);
-            valid = ix < p.W && lrow < p.nrows;
-        }
-        unsigned long long its = 0;
-        if (valid) {
-            uint32_t wre[N], wim[N];
+        if (p.tile_rows_done && !p.list)
+            count_bands(p.W, p.nrows, p.tile_rows_done, p.band_flags, band);
+        bool fresh = false;
+        feed_lanes(
+            feed, !active,
+            [&]() {
+                unsigned t = ~0u;
+                if (lane == 0 && !(p.stop && *p.stop)) {
+                    const unsigned n = atomicAdd(&p.sync->tile_counter, 1u);
+                    if (n < p.tile_limit && p.tile_base + n < total)
+                        t = p.tile_base + n;
+                }
+                return __shfl_sync(0xffffffffu, t, 0);
+            },
+            [&](unsigned t, int& px, int& row) {
+                if (p.list) {
+                    const unsigned i = t * 32u + lane;
+                    const unsigned pix = i < list_n ? p.list[i] : 0u;
+                    row = (int)(pix / (unsigned)p.W);
+                    px = (int)(pix - (unsigned)row * (unsigned)p.W);
+                    return i < list_n;
+                }
+                const int ty = (int)(t / (unsigned)tiles_x);
+                px = (int)(t - (unsigned)ty * (unsigned)tiles_x) * kTileW + (lane & (kTileW - 1));
+                row = ty * kTileH + lane / kTileW;
+                return px < p.W && row < p.nrows;
+            },
+            [&](int k, int px, int row) { tile[warp][k] = make_int2(px, row); },
+            [&](int k) {
+                ix = tile[warp][k].x;
+                lrow = tile[warp][k].y;
+                fresh = true;
+            });
+        if (fresh) {
             const uint32_t* xs = p.xs + (size_t)ix * N;
             const uint32_t* ys = p.ys + (size_t)lrow * N;
 #pragma unroll
             for (int k = 0; k < N; ++k) {
-                wre[k] = xs[k];
-                wim[k] = ys[k];
+                o.wre[k] = xs[k];
+                o.wim[k] = ys[k];
+                c_re.set(k, JULIA ? p.julia[k] : o.wre[k]);
+                c_im.set(k, JULIA ? p.julia[N + k] : o.wim[k]);
             }
-            uint32_t n;
-            float mag = 0.f;
-            if constexpr (c_in_smem<N>()) {
-                const int stride = blockDim.x;
-                uint32_t* cre = smem + threadIdx.x;
-                uint32_t* cim = smem + (size_t)N * stride + threadIdx.x;
-#pragma unroll
-                for (int k = 0; k < N; ++k) {
-                    cre[k * stride] = JULIA ? p.julia[k] : wre[k];
-                    cim[k * stride] = JULIA ? p.julia[N + k] : wim[k];
-                }
-                CShared<N> gr{cre, stride}, gi{cim, stride};
-                n = escape_mp<N, FRACTAL>(wre, wim, gr, gi, p.depth, mag);
-            } else {
-                CRegs<N> gr, gi;
-#pragma unroll
-                for (int k = 0; k < N; ++k) {
-                    gr.w[k] = JULIA ? p.julia[k] : wre[k];
-                    gi.w[k] = JULIA ? p.julia[N + k] : wim[k];
-                }
-                n = escape_mp<N, FRACTAL>(wre, wim, gr, gi, p.depth, mag);
-            }
-            p.out[(size_t)lrow * p.W + ix] = (int32_t)n;
-            if (p.mag)
-                p.mag[(size_t)lrow * p.W + ix] = mag;
-            its = n ? n : p.depth;
+            mp_start<N>(o);
+            active = true;
         }
-        its = warp_sum_u64(its);
-        if (p.band_flags)
-            __threadfence_system();
-        __syncwarp();
-        if (lane == 0) {
-            atomicAdd(&p.sync->iter_sum, its);
-            if (p.tile_rows_done && !p.list) {
-                const unsigned done = atomicAdd(&p.tile_rows_done[ty], 1u) + 1u;
-                if (done == (unsigned)tiles_x && p.band_flags) {
-                    __threadfence_system();
-                    p.band_flags[ty] = 1;
+        if (!__any_sync(0xffffffffu, active))
+            break;
+        // iterate until enough lanes are idle to be worth a look
+        const int enough = (feed.left || feed.more) ? kRefill : 32;
+        do {
+            if (active) {
+                int u = kRefillEvery;
+                bool escaped, done;
+                float mag = 0.f;
+#pragma unroll 1
+                do {
+                    escaped = mp_step<N>(o, c_re, c_im, FRACTAL == MDZ_BURNING_SHIP,
+                                         FRACTAL == MDZ_GENERALIZED_CELTIC, FRACTAL == MDZ_VARIANT,
+                                         o.wz + 1u >= p.depth, mag);
+                    done = escaped || o.wz >= p.depth;
+                } while (!done && --u);
+                if (done) {
+                    const uint32_t n = escaped ? o.wz : 0u;
+                    const size_t at = (size_t)lrow * p.W + ix;
+                    p.out[at] = (int32_t)n;
+                    if (p.mag)
+                        p.mag[at] = mag;
+                    its += n ? n : p.depth;
+                    active = false;
+                    band = lrow / kTileH;
                 }
             }
-        }
+        } while (__popc(__ballot_sync(0xffffffffu, !active)) < enough);
     }
+    its = warp_sum_u64(its);
+    if (lane == 0 && its)
+        atomicAdd(&p.sync->iter_sum, its);
     if (p.done.count)
         done_signal(p.done, (unsigned long long)p.tile_base + p.tile_limit >= total ? 3 : 1);
 }
@@ -304,66 +306,60 @@ __global__ void __launch_bounds__(block_threads<N>()) serve_mp_kernel(ServeDev* 
                 const uint32_t* cxs = rq.julia ? rq.julia : xs;
                 const uint32_t* cys = rq.julia ? rq.julia + N : ys;
                 uint32_t* sp = (uint32_t*)(rq.state + (size_t)pix * rq.state_stride);
-                uint32_t wre[N], wim[N], sre, sim, wz;
+                MpOrbit<N> o;
+                float mag = 0.f;
                 if (e & kEntryFresh) {
 #pragma unroll
                     for (int k = 0; k < N; ++k) {
-                        wre[k] = xs[k];
-                        wim[k] = ys[k];
+                        o.wre[k] = xs[k];
+                        o.wim[k] = ys[k];
                     }
-                    sre = fx::abs_inplace<N>(wre);
-                    sim = fx::abs_inplace<N>(wim);
-                    wz = 1;
+                    mp_start<N>(o);
                 } else {
 #pragma unroll
                     for (int k = 0; k < N; ++k) {
-                        wre[k] = sp[k];
-                        wim[k] = sp[N + k];
+                        o.wre[k] = sp[k];
+                        o.wim[k] = sp[N + k];
                     }
-                    wz = sp[2 * N];
+                    o.wz = sp[2 * N] - 1u;
                     const uint32_t sg = sp[2 * N + 1];
-                    sre = (sg & 1u) ? 0xffffffffu : 0u;
-                    sim = (sg & 2u) ? 0xffffffffu : 0u;
+                    o.sre = (sg & 1u) ? 0xffffffffu : 0u;
+                    o.sim = (sg & 2u) ? 0xffffffffu : 0u;
+                    mp_squares<N>(o, false, mag);
                 }
-                const uint32_t last = wz + d->ctl.budget[slot] - 1u;
                 const uint32_t depth = rq.pl.depth;
-                float mag = 0.f;
-                bool fin;
+                const uint32_t last = min(o.wz + d->ctl.budget[slot], depth);
+                using CGet = typename std::conditional<c_in_smem<N>(), CShared<N>, CRegs<N>>::type;
+                CGet c_re, c_im;
                 if constexpr (c_in_smem<N>()) {
-                    const int stride = blockDim.x;
-                    uint32_t* cre = smem + threadIdx.x;
-                    uint32_t* cim = smem + (size_t)N * stride + threadIdx.x;
-#pragma unroll
-                    for (int k = 0; k < N; ++k) {
-                        cre[k * stride] = cxs[k];
-                        cim[k * stride] = cys[k];
-                    }
-                    CShared<N> gr{cre, stride}, gi{cim, stride};
-                    fin = escape_mp_resume<N>(wre, wim, sre, sim, gr, gi, rq.fractal, wz, last,
-                                              depth, mag);
-                } else {
-                    CRegs<N> gr, gi;
-#pragma unroll
-                    for (int k = 0; k < N; ++k) {
-                        gr.w[k] = cxs[k];
-                        gi.w[k] = cys[k];
-                    }
-                    fin = escape_mp_resume<N>(wre, wim, sre, sim, gr, gi, rq.fractal, wz, last,
-                                              depth, mag);
+                    c_re = CGet{smem + threadIdx.x, (int)blockDim.x};
+                    c_im = CGet{smem + (size_t)N * blockDim.x + threadIdx.x, (int)blockDim.x};
                 }
-                if (fin) {
-                    rq.pl.out[pix] = (int32_t)wz;
+#pragma unroll
+                for (int k = 0; k < N; ++k) {
+                    c_re.set(k, cxs[k]);
+                    c_im.set(k, cys[k]);
+                }
+                const int fr = rq.fractal;
+                bool escaped = false;
+#pragma unroll 1
+                while (!escaped && o.wz < last)
+                    escaped = mp_step<N>(o, c_re, c_im, fr == MDZ_BURNING_SHIP,
+                                         fr == MDZ_GENERALIZED_CELTIC, fr == MDZ_VARIANT,
+                                         o.wz + 1u >= depth, mag);
+                if (escaped || o.wz >= depth) {
+                    rq.pl.out[pix] = escaped ? (int32_t)o.wz : 0;
                     if (rq.pl.mag)
                         rq.pl.mag[pix] = mag;
                     done = true;
                 } else {
 #pragma unroll
                     for (int k = 0; k < N; ++k) {
-                        sp[k] = wre[k];
-                        sp[N + k] = wim[k];
+                        sp[k] = o.wre[k];
+                        sp[N + k] = o.wim[k];
                     }
-                    sp[2 * N] = wz;
-                    sp[2 * N + 1] = (sre & 1u) | (sim & 2u);
+                    sp[2 * N] = o.wz + 1u;
+                    sp[2 * N + 1] = (o.sre & 1u) | (o.sim & 2u);
                     again = true;
                 }
             }
@@ -394,7 +390,7 @@ __global__ void __launch_bounds__(block_threads<N>()) serve_mp_kernel(ServeDev* 
 template <int N, int FRACTAL, bool JULIA>
 int typed_blocks_per_sm(int* out)
 {
-    constexpr int threads = block_threads<N>();
+    constexpr int threads = kFrameBlock;
     const size_t smem = c_in_smem<N>() ? (size_t)2 * N * threads * sizeof(uint32_t) : 0;
     static int blocks_per_sm = 0;
     if (!blocks_per_sm) {
@@ -405,7 +401,7 @@ int typed_blocks_per_sm(int* out)
         int b = 0;
         MDZ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
             &b, mp_frame_kernel<N, FRACTAL, JULIA>, threads, smem));
-        blocks_per_sm = b < 1 ? 1 : b;
+        blocks_per_sm = b < 1 ? 1 : (b < frame_blocks_per_sm<N>() ? b : frame_blocks_per_sm<N>());
     }
     *out = blocks_per_sm;
     return MDZGPU_OK;
@@ -414,7 +410,7 @@ int typed_blocks_per_sm(int* out)
 template <int N, int FRACTAL, bool JULIA>
 int launch_typed(mdzgpu_ctx* ctx, const MpLaunch& p, cudaStream_t s)
 {
-    constexpr int threads = block_threads<N>();
+    constexpr int threads = kFrameBlock;
     const size_t smem = c_in_smem<N>() ? (size_t)2 * N * threads * sizeof(uint32_t) : 0;
     int blocks_per_sm = 1;
     if (int rc = typed_blocks_per_sm<N, FRACTAL, JULIA>(&blocks_per_sm))
