@@ -15,7 +15,7 @@
 // half a cycle.  So an iteration spends three FP64 instructions, all DFMA:
 // the three additions (a + b = fma(a, 1, b); 2 wre wim + c_im in one, the
 // doubling being exact), and forms its three products on the integer pipes,
-// bit for bit as the FP64 pipe would (mul_round); the escape test compares
+// bit for bit as the FP64 pipe would (double_bits.cuh); the escape test compares
 // 20-bit magnitudes and adds in double only near the bailout.  Measured
 // (960x540, 5.4e9 pixel-iterations): 168.6 ms with the nine FP64
 // instructions this replaces and whole tiles, 40.4 ms now; 122 warp
@@ -31,6 +31,9 @@
 // pixel tiles from a global atomic counter, in place of a mutex-protected
 // next_line counter advanced by whole rows, and a lane takes a new pixel as
 // soon as kRefill lanes are idle (pixel_feed.cuh).
+#include <algorithm>
+
+#include "double_bits.cuh"
 #include "internal.h"
 #include "pixel_feed.cuh"
 
@@ -45,81 +48,6 @@ constexpr int kRefillEvery = 4;   // iterations between looks at the idle lanes
 // a boundary point: 40.4 ms with 16 warps, 42.4 with 24, 46.6 with 32, 46.7
 // with 10; refill at 3 idle lanes 40.4 ms, at 6 42.0 ms).
 constexpr int kBlocksPerSm = 4;
-
-// a b + c, never simplified to an addition or a product
-__device__ __forceinline__ double dfma(double a, double b, double c)
-{
-    double r;
-    asm("fma.rn.f64 %0, %1, %2, %3;" : "=d"(r) : "d"(a), "d"(b), "d"(c));
-    return r;
-}
-
-// A double cut in three: its mantissa with the leading 1 (h: top 21 bits,
-// l: low 32) and q = high word - h, its sign and exponent field less one.
-struct Split {
-    uint32_t h, l, q;
-};
-
-__device__ __forceinline__ Split split(double x)
-{
-    const uint32_t hi = (uint32_t)__double2hiint(x);
-    const uint32_t h = (hi & 0x000fffffu) | 0x00100000u;
-    return Split{h, (uint32_t)__double2loint(x), hi - h};
-}
-
-// Whether one of the two has an exponent outside 2^-479 .. 2^32 (0,
-// denormals, infinities and NaN are outside): inside, no product of the two
-// leaves the normal range, and its magnitude fits a float's exponent.  The
-// sign bit falls out of the mask.
-__device__ __forceinline__ bool odd_exponent(const Split& x, const Split& y)
-{
-    const uint32_t lowest = 0x22000000u - 0x00100000u;
-    return (((x.q - lowest) | (y.q - lowest)) & 0x60000000u) != 0u;
-}
-
-// x y rounded to nearest from the product of the mantissas, H 2^64 + m 2^32 +
-// t (t's low word is not needed); q is the sum of the operands' q.  Returns
-// true when the bits below the result's last place are 100..0 as far as m
-// goes: t or the parity decides there, and the caller multiplies in double.
-__device__ __forceinline__ bool round106(uint64_t H, uint64_t m, uint64_t t, uint32_t q,
-                                         uint32_t& hi, uint32_t& lo)
-{
-    uint32_t v, hl, hh;   // bits 32.., 64.., 96.. of the product
-    asm("{add.cc.u32 %0, %3, %4;\n\t"
-        "addc.cc.u32 %1, %5, %6;\n\t"
-        "addc.u32 %2, %7, 0;}"
-        : "=&r"(v), "=&r"(hl), "=r"(hh)
-        : "r"((uint32_t)m), "r"((uint32_t)(t >> 32)), "r"((uint32_t)H), "r"((uint32_t)(m >> 32)),
-          "r"((uint32_t)(H >> 32)));
-    const uint32_t s = hh >> 9;          // 1: the mantissas' product is 2 or more
-    const uint32_t sh = 12u - s;
-    const uint32_t r = v << sh;          // what is rounded away
-    asm("{.reg .u32 c;\n\t"
-        "add.cc.u32 c, %2, %2;\n\t"      // carry = r >> 31: round up
-        "addc.cc.u32 %0, %3, 0;\n\t"
-        "addc.u32 %1, %4, %5;}"
-        : "=&r"(lo), "=r"(hi)
-        : "r"(r), "r"(__funnelshift_l(v, hl, sh)), "r"(__funnelshift_l(hl, hh, sh)),
-          "r"(q + (s << 20) + (0x00200000u - 0x40000000u)));
-    return r == 0x80000000u;
-}
-
-__device__ __forceinline__ uint64_t wide(uint32_t a, uint32_t b)
-{
-    return (uint64_t)a * b;
-}
-
-__device__ __forceinline__ bool mul_round(const Split& x, const Split& y, uint32_t& hi,
-                                          uint32_t& lo)
-{
-    return round106(wide(x.h, y.h), wide(x.h, y.l) + wide(y.h, x.l), wide(x.l, y.l), x.q + y.q, hi,
-                    lo);
-}
-
-__device__ __forceinline__ bool sqr_round(const Split& x, uint32_t& hi, uint32_t& lo)
-{
-    return round106(wide(x.h, x.h), wide(2u * x.h, x.l), wide(x.l, x.l), 2u * x.q, hi, lo);
-}
 
 // A double's high word as a float cut to 20 bits: right for 2^-126 .. 2^128;
 // of a smaller or larger one only the bits' sign and pattern are left.
@@ -271,10 +199,7 @@ __global__ void __launch_bounds__(kBlock) fp64_frame_kernel(Fp64Launch p)
         feed_lanes(
             feed, !active,
             [&]() {
-                unsigned t = 0;
-                if (lane == 0)
-                    t = (p.stop && *p.stop) ? total : atomicAdd(&p.sync->tile_counter, 1u);
-                t = __shfl_sync(0xffffffffu, t, 0);
+                const unsigned t = next_tile(feed, &p.sync->tile_counter, p.stop);
                 return t < total ? t : ~0u;
             },
             [&](unsigned t, int& px, int& row) {
@@ -334,8 +259,9 @@ int launch_one(mdzgpu_ctx* ctx, const Fp64Launch& p, cudaStream_t s)
     }
     const long tiles = (long)((p.W + kTileW - 1) / kTileW) * ((p.nrows + kTileH - 1) / kTileH);
     long grid = (long)ctx->num_sms * (blocks_per_sm < kBlocksPerSm ? blocks_per_sm : kBlocksPerSm);
-    const long warps_needed = tiles;
-    const long blocks_needed = (warps_needed + kBlock / 32 - 1) / (kBlock / 32);
+    // a warp a tile, or fewer; a block an SM as long as there are tiles
+    const long blocks_needed = std::max((tiles + kBlock / 32 - 1) / (kBlock / 32),
+                                        std::min(tiles, (long)ctx->num_sms));
     if (grid > blocks_needed)
         grid = blocks_needed;
     if (grid < 1)

@@ -20,6 +20,7 @@
 //
 // What bounds it is the integer multiplier: N = 10 takes 126 partial products
 // an iteration at 1.1 cycles of an SM each, N = 34 1272 (fixed_point.cuh).
+#include <algorithm>
 #include <type_traits>
 
 #include "fixed_point.cuh"
@@ -185,13 +186,8 @@ __global__ void __launch_bounds__(kFrameBlock, frame_blocks_per_sm<N>())
         feed_lanes(
             feed, !active,
             [&]() {
-                unsigned t = ~0u;
-                if (lane == 0 && !(p.stop && *p.stop)) {
-                    const unsigned n = atomicAdd(&p.sync->tile_counter, 1u);
-                    if (n < p.tile_limit && p.tile_base + n < total)
-                        t = p.tile_base + n;
-                }
-                return __shfl_sync(0xffffffffu, t, 0);
+                const unsigned n = next_tile(feed, &p.sync->tile_counter, p.stop);
+                return n < p.tile_limit && p.tile_base + n < total ? p.tile_base + n : ~0u;
             },
             [&](unsigned t, int& px, int& row) {
                 if (p.list) {
@@ -418,7 +414,8 @@ int launch_typed(mdzgpu_ctx* ctx, const MpLaunch& p, cudaStream_t s)
     const long tiles = p.list ? ((long)p.W * p.nrows + 31) / 32
                               : (long)((p.W + kTileW - 1) / kTileW) * ((p.nrows + kTileH - 1) / kTileH);
     long grid = (long)ctx->num_sms * blocks_per_sm;
-    const long blocks_needed = (tiles + threads / 32 - 1) / (threads / 32);
+    const long blocks_needed = std::max((tiles + threads / 32 - 1) / (threads / 32),
+                                        std::min(tiles, (long)ctx->num_sms));
     if (grid > blocks_needed)
         grid = blocks_needed;
     if (grid < 1)

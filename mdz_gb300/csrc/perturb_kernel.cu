@@ -34,14 +34,14 @@
 // result has |z|^2 > 4, or 0 if none within depth.
 #include <math.h>
 
+#include "double_bits.cuh"
 #include "internal.h"
+#include "pixel_feed.cuh"
 #include "serve.h"
 
 namespace mdz {
 namespace {
 
-constexpr int kTileW = 8;
-constexpr int kTileH = 4;
 // A pixel of the FP32 pass that steps from a reference entry at zero
 // (|Z_m|^2 < 2^-120 for m past the orbit's start: the view is centred on a
 // minibrot's nucleus, Z_p = 0) is handed to the FP64 pass there: around a
@@ -843,9 +843,9 @@ struct Mant<double> {
     static constexpr int kForceSlow = 1000;
     static constexpr double kFoldEps = 3.552713678800501e-15;  // 2^-48
     static constexpr double kEps2x16 = 1.9721522630525295e-31;  // 16 (2^-53)^2
-    __device__ static double scale(double x, int e) { return ldexp(x, e); }
+    __device__ static double scale(double x, int e) { return ldexp_bits(x, e); }
     __device__ static double fma_(double a, double b, double c) { return fma(a, b, c); }
-    __device__ static int exponent_of(double a) { return ilogb(a); }
+    __device__ static int exponent_of(double a) { return ilogb_bits(a); }
 };
 
 template <class T>
@@ -864,7 +864,26 @@ struct PixState {
     T ke;
     T kb;           // 2^18 ke 2^(2e): e2 kb = (2^9 err)^2; 0 when 2^(2e) underflows
     T sm;           // 2^-5 2^e: the fold margin per unit of |t|
+    T tt;           // FP64 pass: ti^2, kept for the next step
 };
+
+// The scale's values as the template below forms them: all are powers of two
+// times a constant, so the FP64 pass takes them from the exponent.
+__device__ __forceinline__ void refresh_scale(PixState<double>& st, double dcm_r, double dcm_i,
+                                              int dce)
+{
+    const int e = st.e;
+    const bool sq = e >= Mant<double>::kSqExp;
+    st.s = ldexp_bits(1.0, e);
+    st.s2scr = sq ? ldexp_bits(1.0000152587890625, 2 * e) : 0.0;
+    st.dcr = ldexp_bits(dcm_r, dce - e);
+    st.dci = ldexp_bits(dcm_i, dce - e);
+    st.slow_if_tiny = e < Mant<double>::kSlowExp;
+    st.force_slow = (dcm_r != 0.0 || dcm_i != 0.0) && (dce - e) > Mant<double>::kForceSlow;
+    st.careful = st.slow_if_tiny || st.force_slow;
+    st.kb = sq ? ldexp_bits(st.ke, 2 * e + 18) : 0.0;
+    st.sm = ldexp_bits(0.03125, e);
+}
 
 template <class T>
 __device__ __forceinline__ void refresh_scale(PixState<T>& st, T dcm_r, T dcm_i, int dce)
@@ -890,18 +909,21 @@ __device__ __forceinline__ void set_from_double(PixState<T>& st, double xr, doub
     if (a == 0.0) {
         st.tr = (T)0;
         st.ti = (T)0;
+        st.tt = (T)0;
         st.e = E;
         return;
     }
-    const int k = ilogb(a);
-    st.tr = (T)ldexp(xr, -k);
-    st.ti = (T)ldexp(xi, -k);
+    const int k = ilogb_bits(a);
+    st.tr = (T)ldexp_bits(xr, -k);
+    st.ti = (T)ldexp_bits(xi, -k);
     st.e = E + k;
+    if constexpr (sizeof(T) == 8)
+        st.tt = st.ti * st.ti;
 }
 
 __device__ __forceinline__ int dexp_of(double x)
 {
-    return x == 0.0 ? -100000 : ilogb(x);
+    return x == 0.0 ? -100000 : ilogb_bits(x);
 }
 
 // ---- rare paths, kept out of the hot loop's instruction stream ----
@@ -918,8 +940,8 @@ __device__ __forceinline__ bool rebase_fp64(const PerturbLaunch& p, int m, PixSt
     const double2 zd = p.zd[m];
     const int ze = p.ze[m];
     const int E = max(dexp_of(fmax(fabs(zd.x), fabs(zd.y))) + ze, st.e + 40);
-    const double dr = ldexp((double)st.tr, st.e - E), di = ldexp((double)st.ti, st.e - E);
-    const double fr = ldexp(zd.x, ze - E) + dr, fi = ldexp(zd.y, ze - E) + di;
+    const double dr = ldexp_bits((double)st.tr, st.e - E), di = ldexp_bits((double)st.ti, st.e - E);
+    const double fr = ldexp_bits(zd.x, ze - E) + dr, fi = ldexp_bits(zd.y, ze - E) + di;
     const double z2 = fr * fr + fi * fi, d2 = dr * dr + di * di;
     if (only_if_glitch && !(z2 < d2))
         return false;
@@ -945,8 +967,8 @@ __device__ __forceinline__ void slow_step(const PerturbLaunch& p, int m, PixStat
     const int E = max(max(dexp_of(fmax(fabs(ar), fabs(ai))) + ae,
                           dexp_of(fmax(fabs(br), fabs(bi))) + be),
                       dexp_of(fmax(fabs(dcm_r), fabs(dcm_i))) + dce);
-    const double rr = ldexp(ar, ae - E) + ldexp(br, be - E) + ldexp(dcm_r, dce - E);
-    const double ri = ldexp(ai, ae - E) + ldexp(bi, be - E) + ldexp(dcm_i, dce - E);
+    const double rr = ldexp_bits(ar, ae - E) + ldexp_bits(br, be - E) + ldexp_bits(dcm_r, dce - E);
+    const double ri = ldexp_bits(ai, ae - E) + ldexp_bits(bi, be - E) + ldexp_bits(dcm_i, dce - E);
     set_from_double(st, rr, ri, E);
     refresh_scale(st, dcf_r, dcf_i, dce);
 }
@@ -970,7 +992,7 @@ __device__ __forceinline__ bool escape_exact(const PerturbLaunch& p, int m, cons
     const double t3 = (double)st.tr * st.tr + (double)st.ti * st.ti;
     const int e3 = 2 * st.e;
     const int E = max(max(dexp_of(dd) + de, dexp_of(t2) + e2), dexp_of(t3) + e3);
-    const double v = ldexp(dd, de - E) + ldexp(t2, e2 - E) + ldexp(t3, e3 - E);
+    const double v = ldexp_bits(dd, de - E) + ldexp_bits(t2, e2 - E) + ldexp_bits(t3, e3 - E);
     return v > 0.0;
 }
 
@@ -1005,6 +1027,16 @@ __device__ __forceinline__ bool four_not_tiny(const PerturbLaunch& p, int m)
     return (__funnelshift_r(lo, hi, (unsigned)m & 31u) & 0xfu) == 0u;
 }
 
+// |z|^2 as the pixel loop forms it.
+__device__ __forceinline__ float mag2(float zr, float zi)
+{
+    return fmaf(zr, zr, zi * zi);
+}
+__device__ __forceinline__ double mag2(double zr, double zi)
+{
+    return fma(zr, zr, sqr_bits(zi));
+}
+
 template <class T>
 __device__ __forceinline__ void load_z(const PerturbLaunch& p, int m, T& zx, T& zy)
 {
@@ -1015,8 +1047,8 @@ __device__ __forceinline__ void load_z(const PerturbLaunch& p, int m, T& zx, T& 
     } else {
         const double2 zd = p.zd[m];
         const int ze = p.ze[m];
-        zx = (T)(ze ? ldexp(zd.x, ze) : zd.x);
-        zy = (T)(ze ? ldexp(zd.y, ze) : zd.y);
+        zx = (T)(ze ? ldexp_bits(zd.x, ze) : zd.x);
+        zy = (T)(ze ? ldexp_bits(zd.y, ze) : zd.y);
     }
 }
 
@@ -1058,6 +1090,30 @@ __device__ __forceinline__ bool fold_certain(T zr, T zi, T Zx, T Zy, T fs, T dzm
     return fs * (ar - ai) > Mant<T>::fma_(eps, ar + ai, dzm + dzm);
 }
 
+// fold_certain of the FP64 pass, from the high words where they show it; hd is
+// the high word of dz's larger component (0 once the estimate is lost).
+template <int FR>
+__device__ __forceinline__ bool fold_certain_bits(double zr, double zi, double Zx, double Zy,
+                                                  double fs, int hd)
+{
+    const int hr = hi_of(zr) & 0x7fffffff, hi = hi_of(zi) & 0x7fffffff;
+    if (FR == MDZ_BURNING_SHIP) {
+        // eps = 2^-48, and 2^-5 |dz|, with a binade to spare
+        const int d = max(hd - (3 << 20), 1 << 20);
+        return (hi_of(zr) ^ hi_of(zi) ^ hi_of(fs)) >= 0
+               && hr > max((hi_of(Zx) & 0x7fffffff) - (46 << 20), d)
+               && hi > max((hi_of(Zy) & 0x7fffffff) - (46 << 20), d);
+    }
+    // |zr|, |zi| and dz as floats cut to 20 bits, where they are in range
+    if ((unsigned)(max(hr, hi) - 0x39000000) > 0x0e000000u || hd > 0x47000000)
+        return false;
+    const float ar = __int_as_float(max(hr - 0x38000000, 0) << 3);
+    const float ai = __int_as_float(max(hi - 0x38000000, 0) << 3);
+    const float dz = __int_as_float(max(hd - 0x38000000, 0) << 3);
+    const float side = hi_of(fs) < 0 ? ai - ar : ar - ai;
+    return side > 4e-6f * (ar + ai) + 0.07f * dz;
+}
+
 // Error estimate of the folded formulas' deltas.  Every step rounds t
 // (inj <= 4 eps |t'|), and the step's Jacobian in t is 2 z (times a
 // reflection where a component is folded), so an error grows by |2 z| a
@@ -1076,11 +1132,98 @@ __device__ __forceinline__ T fold_ke(const PerturbLaunch&)
     return (T)(Mant<T>::kEps2x16 * 16.0);
 }
 
-template <class T>
-__device__ __forceinline__ bool fold_err_hopeless(const PixState<T>& st)
+__device__ __forceinline__ bool fold_err_hopeless(const PixState<float>& st)
 {
-    const T dd = Mant<T>::fma_(st.tr, st.tr, st.ti * st.ti);
-    return !(st.ke * st.e2 <= (T)1.52587890625e-05 * dd) || !(st.kb * st.e2 <= (T)0.015625);
+    const float dd = fmaf(st.tr, st.tr, st.ti * st.ti);
+    return !(st.ke * st.e2 <= 1.52587890625e-05f * dd) || !(st.kb * st.e2 <= 0.015625f);
+}
+
+// The FP64 pass decides from exponents where it can: the high words of two
+// positive doubles, added, are 1023 + log2 of their product (in units of
+// 2^-20) less at most 0.18.
+__device__ __forceinline__ unsigned log_sum(double a, double b)
+{
+    return (unsigned)hi_of(a) + (unsigned)hi_of(b);
+}
+
+__device__ __forceinline__ bool fold_err_hopeless(const PixState<double>& st)
+{
+    const double dd = fma(st.tr, st.tr, st.tt);
+    const unsigned d = (unsigned)hi_of(dd);
+    // ke e2 < 2^-17 dd and kb e2 < 2^-6.8
+    if ((unsigned)hi_of(st.e2) < 0x60000000u && d < 0x7ff00000u
+        && log_sum(st.ke, st.e2) - 0x3ff00000u + (17u << 20) < d
+        && log_sum(st.kb, st.e2) < 0x3ff00000u + 0x3f800000u)
+        return false;
+    bool r;
+    do
+        r = !(mul_here(st.ke, st.e2) <= mul_here(1.52587890625e-05, dd))
+            || !(mul_here(st.kb, st.e2) <= 0.015625);
+    while (once());
+    return r;
+}
+
+// Within reach of the bailout: |z|^2 > 4 - 2^-14, or nearer to 4 than 2^9
+// times the error estimate of z.
+__device__ __forceinline__ bool near_bailout(float mag, const PixState<float>& st, bool lost_track)
+{
+    const float dv = mag - 4.f;
+    return dv > -6.1035156e-5f || (!lost_track && dv * dv <= st.kb * st.e2);
+}
+
+__device__ __forceinline__ bool near_bailout(double mag, const PixState<double>& st,
+                                             bool lost_track)
+{
+    // |z|^2 < 3.875 and kb e2 < 2^-14.8 < 0.125^2
+    if ((unsigned)hi_of(mag) < 0x400f0000u
+        && (lost_track || log_sum(st.kb, st.e2) < 0x3ff00000u + 0x3f000000u))
+        return false;
+    bool r;
+    do {
+        const double dv = add_here(mag, -4.0);
+        r = dv > -6.1035156e-5 || (!lost_track && mul_here(dv, dv) <= mul_here(st.kb, st.e2));
+    } while (once());
+    return r;
+}
+
+// The rebase screen |z|^2 <= (1 + 2^-16) |dz|^2 or |z| tiny (dd = |t|^2).
+__device__ __forceinline__ bool rebase_screen(float mag, float dd, const PixState<float>& st)
+{
+    return fmaf(st.s2scr, dd, -mag) >= 0.f || mag < Mant<float>::kGlitchZ2;
+}
+
+__device__ __forceinline__ bool rebase_screen(double mag, double dd, const PixState<double>& st)
+{
+    // |z|^2 >= 2^-59 and, by the high words, above (1 + 2^-16) dd 2^(2e)
+    const int m = hi_of(mag);
+    if (m >= 0x3c400000 && hi_of(dd) + max(st.e, -512) * (1 << 21) + 64 < m)
+        return false;
+    bool r;
+    do
+        r = fma_here(st.s2scr, dd, -mag) >= 0.0 || mag < Mant<double>::kGlitchZ2;
+    while (once());
+    return r;
+}
+
+// |t| outside [2^-32, 2^32] (and not 0); k is its exponent when it is.
+template <class T>
+__device__ __forceinline__ bool needs_rescale(T tr, T ti, int& k)
+{
+    if constexpr (sizeof(T) == 8) {
+        // the high words decide but for those of the two limits
+        const int h = max(hi_of(tr) & 0x7fffffff, hi_of(ti) & 0x7fffffff);
+        if ((unsigned)(h - 0x3df00000) < 0x04000000u)
+            return false;
+        if (h != 0x41f00000 && h != 0x3defffff && h >= 0x00100000 && h < 0x7ff00000) {
+            k = (h >> 20) - 1023;
+            return true;
+        }
+    }
+    const T amax = fmax(fabs(tr), fabs(ti));
+    if (!((amax > (T)4.2949673e9 || amax < (T)2.3283064e-10) && amax != (T)0))
+        return false;
+    k = Mant<T>::exponent_of(amax);
+    return true;
 }
 
 // The every-4th-iteration check.  A trajectory whose estimate passed the
@@ -1115,8 +1258,8 @@ __device__ __forceinline__ void fold_rebase_err(const PerturbLaunch& p, int m, P
     const double2 zd = p.zd[m];
     const int ze = p.ze[m];
     const double z2 = zd.x * zd.x + zd.y * zd.y;
-    const double add = ldexp(z2 * 4.930380657631324e-32 / (double)st.ke, 2 * (ze - st.e));
-    st.e2 = (T)(ldexp((double)st.e2, 2 * (e0 - st.e)) + add);   // 2^-104 |Z|^2 above
+    const double add = ldexp_bits(z2 * 4.930380657631324e-32 / (double)st.ke, 2 * (ze - st.e));
+    st.e2 = (T)(ldexp_bits((double)st.e2, 2 * (e0 - st.e)) + add);   // 2^-104 |Z|^2 above
 }
 
 // |z|^2 > 4 for a folded formula, exactly as escape_exact; `unsure` when
@@ -1133,9 +1276,9 @@ __device__ bool escape_fold(const PerturbLaunch& p, int m, const PixState<T>& st
     const double t3 = (double)st.tr * st.tr + (double)st.ti * st.ti;
     const int e3 = 2 * st.e;
     const int E = max(max(dexp_of(dd) + de, dexp_of(t2) + e2), dexp_of(t3) + e3);
-    const double v = ldexp(dd, de - E) + ldexp(t2, e2 - E) + ldexp(t3, e3 - E);
-    const double margin = ldexp(v, E);
-    const double err = ldexp(sqrt((double)st.ke * (double)st.e2), st.e);
+    const double v = ldexp_bits(dd, de - E) + ldexp_bits(t2, e2 - E) + ldexp_bits(t3, e3 - E);
+    const double margin = ldexp_bits(v, E);
+    const double err = ldexp_bits(sqrt((double)st.ke * (double)st.e2), st.e);
     unsure = !(fabs(margin) > err * (4.5 + err));
     return v > 0.0;
 }
@@ -1178,22 +1321,22 @@ __device__ __forceinline__ void fold_step(const PerturbLaunch& p, int m, PixStat
     if (FR == MDZ_BURNING_SHIP) {
         const int Ex = max(dexp_of(zd.x) + ze, dexp_of(tr) + st.e);
         const int Ey = max(dexp_of(zd.y) + ze, dexp_of(ti) + st.e);
-        const double xr = ldexp(zd.x, ze - Ex) + ldexp(tr, st.e - Ex);
-        const double xi = ldexp(zd.y, ze - Ey) + ldexp(ti, st.e - Ey);
+        const double xr = ldexp_bits(zd.x, ze - Ex) + ldexp_bits(tr, st.e - Ex);
+        const double xi = ldexp_bits(zd.y, ze - Ey) + ldexp_bits(ti, st.e - Ey);
         side = ((xr < 0.0) != (xi < 0.0)) ? -1.0 : 1.0;
-        sure = fabs(xr) > fmax(eps, ldexp(ea, st.e - Ex))
-               && fabs(xi) > fmax(eps, ldexp(ea, st.e - Ey));
+        sure = fabs(xr) > fmax(eps, ldexp_bits(ea, st.e - Ex))
+               && fabs(xi) > fmax(eps, ldexp_bits(ea, st.e - Ey));
     } else {
         const int Es = max(max(dexp_of(fmax(fabs(ar), fabs(ai))) + ae,
                                dexp_of(fmax(fabs(br), fabs(bi))) + be),
                            dexp_of(fmv) + fev);
-        const double cs = ldexp(fmv, fev - Es);
-        const double a1 = ldexp(ar, ae - Es), b1 = ldexp(br, be - Es);
+        const double cs = ldexp_bits(fmv, fev - Es);
+        const double a1 = ldexp_bits(ar, ae - Es), b1 = ldexp_bits(br, be - Es);
         const double v = cs + (a1 + b1);
         side = v < 0.0 ? -1.0 : 1.0;
         // | |x|^2 - |y|^2 | moves by at most 2 sqrt2 |z| err + 2 err^2
         sure = fabs(v) > eps * (fabs(cs) + fabs(a1) + fabs(b1))
-               && fabs(v) > ldexp(ea, st.e - Es) * (6.0 + ldexp(ea, st.e));
+               && fabs(v) > ldexp_bits(ea, st.e - Es) * (6.0 + ldexp_bits(ea, st.e));
     }
     if (!sure)
         lost += 64.f;  // undecidable here: the next pass redoes it
@@ -1210,17 +1353,17 @@ __device__ __forceinline__ void fold_step(const PerturbLaunch& p, int m, PixStat
     double rr, ri;
     if (FR == MDZ_BURNING_SHIP) {
         // Re: unfolded; Im: 2 (|c + d| - |c|) with d = Z_re dz_im + dz_re Z_im + dz_re dz_im
-        rr = ldexp(ar, ae - E) + ldexp(br, be - E) + ldexp(dcm_r, dce - E);
-        const double dd2 = ldexp(ai, ae - E) + ldexp(bi, be - E);   // = 2 d
-        fi_ = cross ? -sc * (ldexp(fmv, fev + 2 - E) + dd2) : sc * dd2;
-        ri = fi_ + ldexp(dcm_i, dce - E);
+        rr = ldexp_bits(ar, ae - E) + ldexp_bits(br, be - E) + ldexp_bits(dcm_r, dce - E);
+        const double dd2 = ldexp_bits(ai, ae - E) + ldexp_bits(bi, be - E);   // = 2 d
+        fi_ = cross ? -sc * (ldexp_bits(fmv, fev + 2 - E) + dd2) : sc * dd2;
+        ri = fi_ + ldexp_bits(dcm_i, dce - E);
         (void)fr_;
     } else {
         // Re: |c + d| - |c| with d = 2 Re(Z dz) + Re(dz^2); Im: unfolded
-        const double d = ldexp(ar, ae - E) + ldexp(br, be - E);
-        fr_ = cross ? -sc * (ldexp(fmv, fev + 1 - E) + d) : sc * d;
-        rr = fr_ + ldexp(dcm_r, dce - E);
-        ri = ldexp(ai, ae - E) + ldexp(bi, be - E) + ldexp(dcm_i, dce - E);
+        const double d = ldexp_bits(ar, ae - E) + ldexp_bits(br, be - E);
+        fr_ = cross ? -sc * (ldexp_bits(fmv, fev + 1 - E) + d) : sc * d;
+        rr = fr_ + ldexp_bits(dcm_r, dce - E);
+        ri = ldexp_bits(ai, ae - E) + ldexp_bits(bi, be - E) + ldexp_bits(dcm_i, dce - E);
         (void)fi_;
     }
     set_from_double(st, rr, ri, E);
@@ -1313,9 +1456,24 @@ __device__ __forceinline__ void pixel_start(PixRun<T>& r, double dcm_r, double d
 #ifndef MDZ_STEP_VARIANT
 #define MDZ_STEP_VARIANT 2
 #endif
-template <class T>
-__device__ __forceinline__ void fast_step(PixState<T>& st, T Zx, T Zy, T zr, T zi)
+// The FP64 pass's step, with fewer FP64 instructions for the same values: 2 Z
+// (2 ti) terms as (2 Z) t, ti^2 kept from the last step's |t|^2, and the
+// product on the integer pipes.
+__device__ __forceinline__ void fast_step(PixState<double>& st, double Zx, double Zy, double,
+                                          double)
 {
+    const double tr = st.tr, ti = st.ti;
+    const double X = times_pow2<1>(Zx), Y = times_pow2<1>(Zy);
+    const double a = fma(tr, tr, -st.tt);
+    const double b = mul2_bits(tr, ti);
+    st.tr = fma(X, tr, fma(-Y, ti, fma(st.s, a, st.dcr)));
+    st.ti = fma(X, ti, fma(Y, tr, fma(st.s, b, st.dci)));
+}
+
+__device__ __forceinline__ void fast_step(PixState<float>& st, float Zx, float Zy, float zr,
+                                          float zi)
+{
+    using T = float;
     const T tr = st.tr, ti = st.ti;
 #if MDZ_STEP_VARIANT == 0
     const T wr = zr + Zx, wi = zi + Zy;
@@ -1342,6 +1500,20 @@ template <class T, int FR>
 __device__ __forceinline__ void fold_fast_step(PixState<T>& st, T Zx, T Zy, T fs)
 {
     const T tr = st.tr, ti = st.ti;
+    if constexpr (sizeof(T) == 8) {
+        // as fast_step's FP64 form
+        const double X = times_pow2<1>(Zx), Y = times_pow2<1>(Zy);
+        const double a = fma(tr, tr, -st.tt);
+        const double b = mul2_bits(tr, ti);
+        if (FR == MDZ_BURNING_SHIP) {
+            st.tr = fma(X, tr, fma(-Y, ti, fma(st.s, a, st.dcr)));
+            st.ti = fma(fs, fma(X, ti, fma(Y, tr, st.s * b)), st.dci);
+        } else {
+            st.tr = fma(fs, fma(X, tr, fma(-Y, ti, st.s * a)), st.dcr);
+            st.ti = fma(X, ti, fma(Y, tr, fma(st.s, b, st.dci)));
+        }
+        return;
+    }
     const T u = tr + tr, v = ti + ti;
     const T a = Mant<T>::fma_(tr, tr, -ti * ti);
     const T b = tr * v;
@@ -1420,14 +1592,19 @@ __device__ __forceinline__ FPair fp_twice(FPair a)
 // needs once z is far from the reference.  The iteration runs in float
 // pairs (~48 bits; FP64 would resolve such an orbit no better, its error
 // having already passed the estimate's limit, and costs ~6x the issue
-// time).  z = z_wz; runs iterations wz + 1 .. depth.  Returns the count
-// (0: did not escape).
+// time).  The state is z after iteration wz; runs iterations wz + 1 .. depth.
+// Returns the count (0: did not escape).
+struct DirectPixel {
+    FPair xr, xi, cr, ci;
+    uint32_t wz, pix;
+};
+
 template <int FR>
-__device__ uint32_t fold_direct(double xr0, double xi0, double cr0, double ci0, uint32_t wz,
-                                uint32_t depth, float& mag)
+__device__ uint32_t fold_direct(const DirectPixel& q, uint32_t depth, float& mag)
 {
-    FPair xr = fp_from(xr0), xi = fp_from(xi0);
-    const FPair cr = fp_from(cr0), ci = fp_from(ci0);
+    FPair xr = q.xr, xi = q.xi;
+    const FPair cr = q.cr, ci = q.ci;
+    const uint32_t wz = q.wz;
     for (uint32_t w = wz + 1; w <= depth; ++w) {
         const FPair x2 = fp_mul(xr, xr), y2 = fp_mul(xi, xi);
         const FPair a = fp_add(x2, fp_neg(y2));
@@ -1478,7 +1655,9 @@ __device__ __forceinline__ OrbitSnap orbit_snapshot(const PerturbLaunch& p)
 // Iterations r.wz .. wz_last (inclusive, <= depth).  Returns 1 when the
 // pixel is finished (*count = escape iteration, or 0 at depth), 0 when it
 // stopped after wz_last or (snapshot mode) at the last finished orbit entry
-// (state in r), -1 when an orbit wait gave up.
+// (state in r), -1 when an orbit wait gave up, 2 (FP64 pass, folded formulas)
+// when the error estimate was lost after iteration r.wz with z in r.st.tr,
+// r.st.ti (fold_direct iterates on).
 //
 // One iteration (dz = t 2^e, s = 2^e, z = Z_m + dz):
 //   w  = z + Z_m                        (= 2 Z_m + s t; z carried from the
@@ -1548,12 +1727,13 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
     float lost_sink = 0.f;
     float& rebase_lost = kTrack ? lost_sink : r.lost;
     if (kTrack)
-        magT = Mant<T>::fma_(zr, zr, zi * zi);
+        magT = mag2(zr, zi);
     const uint32_t last = wz_last < p.depth ? wz_last : p.depth;
     uint32_t wz = r.wz;
     bool blocked = false;
     while (wz <= last) {
         bool attention = false;
+        T dd;   // |t|^2 after the step
         // blocks: FP32 (the FP64 pass is the rare escalation path), no
         // slow step among the four (dz below the FP32 range needs one only
         // where Z_m is tiny)
@@ -1726,7 +1906,7 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
             } else {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    fast_step<T>(st, Zx, Zy, zr, zi);
+                    fast_step(st, Zx, Zy, zr, zi);
                     ++m;
                     load_z<T>(p, m, Zx, Zy);
                     zr = Mant<T>::fma_(st.s, st.tr, Zx);
@@ -1781,7 +1961,7 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
                     zr = Mant<T>::fma_(st.s, st.tr, Zx);
                     zi = Mant<T>::fma_(st.s, st.ti, Zy);
                     if (kTrack)
-                        magT = Mant<T>::fma_(zr, zr, zi * zi);
+                        magT = mag2(zr, zi);
                     ++r.rebases;
                 }
             }
@@ -1798,19 +1978,38 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
                     return 1;
                 }
             }
-            const T g = kTrack ? grow * magT : (T)0;
+            T g = (T)0;
+            if constexpr (sizeof(T) == 8)
+                g = times_pow2<2>(magT);
+            else if (kTrack)
+                g = grow * magT;
             // the hybrid folds on odd iterations only
             if (FR != MDZ_MANDELBROT && (!kVar || (wz & 1u))) {
                 // with dz below the T range (s = 0) a fold is out of reach
                 // unless the entry is marked: the same choice as the blocks
                 // (a lost estimate leaves only the rounding margin: the side
                 // is still decided exactly, its error no longer matters)
-                const bool fast =
-                    !careful && !axis_bit(p, m)
-                    && (st.s == (T)0
-                        || fold_certain<T, FR>(
-                            zr, zi, Zx, Zy, fs,
-                            lost_track ? (T)0 : st.sm * fmax(fabs(st.tr), fabs(st.ti))));
+                bool fast = !careful && !axis_bit(p, m);
+                if constexpr (sizeof(T) == 8) {
+                    const int hd = lost_track ? 0
+                                              : max(hi_of(st.tr) & 0x7fffffff,
+                                                    hi_of(st.ti) & 0x7fffffff)
+                                                    + st.e * (1 << 20);
+                    if (fast && !(st.s == (T)0)
+                        && !fold_certain_bits<FR>(zr, zi, Zx, Zy, fs, hd)) {
+                        do {
+                            const T dzm = mul_here(st.sm, fmax(fabs(st.tr), fabs(st.ti)));
+                            fast = fold_certain<T, FR>(zr, zi, Zx, Zy, fs,
+                                                       lost_track ? (T)0 : dzm);
+                        } while (once());
+                    }
+                } else {
+                    fast = fast
+                           && (st.s == (T)0
+                               || fold_certain<T, FR>(
+                                   zr, zi, Zx, Zy, fs,
+                                   lost_track ? (T)0 : st.sm * fmax(fabs(st.tr), fabs(st.ti))));
+                }
                 if (fast) {
                     fold_fast_step<T, FR>(st, Zx, Zy, fs);
                 } else {
@@ -1828,7 +2027,7 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
                 if (kTrack && st.e != e0)
                     st.e2 = Mant<T>::scale(st.e2, 2 * (e0 - st.e));
             } else {
-                fast_step<T>(st, Zx, Zy, zr, zi);
+                fast_step(st, Zx, Zy, zr, zi);
             }
             ++m;
             load_z<T>(p, m, Zx, Zy);
@@ -1836,15 +2035,20 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
                 fs = (T)fold_sign(p, m);
             zr = Mant<T>::fma_(st.s, st.tr, Zx);
             zi = Mant<T>::fma_(st.s, st.ti, Zy);
-            magT = Mant<T>::fma_(zr, zr, zi * zi);
+            magT = mag2(zr, zi);
+            if constexpr (sizeof(T) == 8) {
+                st.tt = sqr_bits(st.ti);
+                dd = Mant<T>::fma_(st.tr, st.tr, st.tt);
+            } else {
+                dd = Mant<T>::fma_(st.tr, st.tr, st.ti * st.ti);
+            }
             if (kTrack)
-                st.e2 = Mant<T>::fma_(g, st.e2, Mant<T>::fma_(st.tr, st.tr, st.ti * st.ti));
+                st.e2 = Mant<T>::fma_(g, st.e2, dd);
         }
         if (kTrack) {
             // the band widens to 2^9 err where the error estimate of z is
             // larger (not once the estimate is lost: its decisions stand)
-            const T dv = magT - (T)4;
-            if (dv > -(T)6.1035156e-5 || (!lost_track && dv * dv <= st.kb * st.e2)) {
+            if (near_bailout(magT, st, lost_track)) {
                 bool unsure;
                 const bool esc = escape_fold<T>(p, m, st, unsure);
                 if (unsure && !lost_track)
@@ -1871,8 +2075,9 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
         // test would not rebase either.  (Once a pixel has left the
         // reference, |z| and |dz| are alike in size and a screen as loose
         // as |z| <= 2 |dz| sent most of its steps through FP64.)
-        const T dd = Mant<T>::fma_(st.tr, st.tr, st.ti * st.ti);
-        if (Mant<T>::fma_(st.s2scr, dd, -magT) >= (T)0 || magT < (T)Mant<T>::kGlitchZ2) {
+        if (sizeof(T) == 4)
+            dd = Mant<T>::fma_(st.tr, st.tr, st.ti * st.ti);
+        if (rebase_screen(magT, dd, st)) {
             const int e0 = st.e;
             if (rebase_fp64<T>(p, m, st, dcf_r, dcf_i, dce, rebase_lost, true)) {
                 if (kTrack)
@@ -1886,7 +2091,7 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
                 zr = Mant<T>::fma_(st.s, st.tr, Zx);
                 zi = Mant<T>::fma_(st.s, st.ti, Zy);
                 if (kTrack)
-                    magT = Mant<T>::fma_(zr, zr, zi * zi);
+                    magT = mag2(zr, zi);
                 ++r.rebases;
                 ++wz;
                 continue;
@@ -1895,12 +2100,17 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
         // keep |t| in [2^-32, 2^32]; it changes by at most ~2^3 a step, so
         // checking every 4th step is enough
         if ((wz & 3u) == 0u) {
-            const T amax = fmax(fabs(st.tr), fabs(st.ti));
-            if ((amax > (T)4.2949673e9 || amax < (T)2.3283064e-10) && amax != (T)0) {
-                const int k = Mant<T>::exponent_of(amax);
+            int k;
+            if (needs_rescale(st.tr, st.ti, k)) {
                 const T sc = Mant<T>::scale((T)1, -k);
-                st.tr *= sc;
-                st.ti *= sc;
+                if constexpr (sizeof(T) == 8) {
+                    st.tr = ldexp_bits(st.tr, -k);
+                    st.ti = ldexp_bits(st.ti, -k);
+                    st.tt = sqr_bits(st.ti);
+                } else {
+                    st.tr *= sc;
+                    st.ti *= sc;
+                }
                 st.e += k;
                 if (kTrack)
                     st.e2 = Mant<T>::scale(st.e2, -2 * k);
@@ -1913,17 +2123,12 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
                 count = 0;
                 return 1;  // the next pass redoes the pixel
             }
-            if (FR != MDZ_MANDELBROT && sizeof(T) == 8 && MODE == kOrbitComplete && lost_track
-                && last == p.depth) {
-                // c = Z_1 + dc
-                const double cr = ldexp(p.zd[1].x, p.ze[1]) + ldexp(dcm_r, dce);
-                const double ci = ldexp(p.zd[1].y, p.ze[1]) + ldexp(dcm_i, dce);
-                float mg = 0.f;
-                count = fold_direct<FR>((double)zr, (double)zi, cr, ci, wz, p.depth, mg);
-                r.mag = mg;
-                r.m = m;
-                r.wz = p.depth + 1;
-                return 1;
+            if (FR != MDZ_MANDELBROT && sizeof(T) == 8 && lost_track) {
+                // the caller iterates the rest directly, from z after wz
+                st.tr = zr;
+                st.ti = zi;
+                r.wz = wz;
+                return 2;
             }
         }
         ++wz;
@@ -1975,11 +2180,10 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
     return v;
 }
 
-// Frame pass (FP32): 8x4 tiles per warp from the atomic counter.  Pass 2
-// (FP64) walks the list of pixels the previous pass flagged, in warp-sized
-// chunks.  Each pass appends the pixels it could not finish precisely to
-// p.flag_out; pixel-iterations are counted only for pixels it finalises.
-template <class T, bool WANT_MAG, bool LIST, bool STREAM, int FR, bool JU = false>
+// Frame pass (FP32): 8x4 tiles per warp from the atomic counter.  Each pass
+// appends the pixels it could not finish precisely to p.flag_out;
+// pixel-iterations are counted only for pixels it finalises.
+template <class T, bool WANT_MAG, bool STREAM, int FR, bool JU = false>
 __device__ __forceinline__ void pixel_tiles(const PerturbLaunch& p)
 {
     __shared__ BlockOrbitView view;
@@ -1994,9 +2198,7 @@ __device__ __forceinline__ void pixel_tiles(const PerturbLaunch& p)
     const int lane = threadIdx.x & 31;
     const int tiles_x = (p.W + kTileW - 1) / kTileW;
     const int tiles_y = (p.nrows + kTileH - 1) / kTileH;
-    const unsigned total = LIST ? (unsigned)((*p.list_in_count + 31) / 32)
-                                : (unsigned)tiles_x * (unsigned)tiles_y;
-    const unsigned list_n = LIST ? *p.list_in_count : 0u;
+    const unsigned total = (unsigned)tiles_x * (unsigned)tiles_y;
     for (;;) {
         unsigned tile = 0;
         if (lane == 0) {
@@ -2007,21 +2209,11 @@ __device__ __forceinline__ void pixel_tiles(const PerturbLaunch& p)
         tile = __shfl_sync(0xffffffffu, tile, 0);
         if (tile >= total)
             break;
-        int ix, lrow;
-        bool valid;
-        if (LIST) {
-            const unsigned i = tile * 32u + lane;
-            valid = i < list_n;
-            const unsigned pix = valid ? p.list_in[i] : 0u;
-            lrow = (int)(pix / (unsigned)p.W);
-            ix = (int)(pix - (unsigned)lrow * (unsigned)p.W);
-        } else {
-            const int ty = (int)(tile / (unsigned)tiles_x);
-            const int tx = (int)(tile - (unsigned)ty * (unsigned)tiles_x);
-            ix = tx * kTileW + (lane & (kTileW - 1));
-            lrow = ty * kTileH + (lane / kTileW);
-            valid = ix < p.W && lrow < p.nrows;
-        }
+        const int ty = (int)(tile / (unsigned)tiles_x);
+        const int tx = (int)(tile - (unsigned)ty * (unsigned)tiles_x);
+        const int ix = tx * kTileW + (lane & (kTileW - 1));
+        const int lrow = ty * kTileH + (lane / kTileW);
+        const bool valid = ix < p.W && lrow < p.nrows;
         unsigned long long its = 0;
         unsigned reb = 0;
         if (valid) {
@@ -2054,10 +2246,145 @@ __device__ __forceinline__ void pixel_tiles(const PerturbLaunch& p)
     }
 }
 
-template <class T, bool WANT_MAG, bool LIST, int FR, bool JU>
-__global__ void __launch_bounds__(256) perturb_kernel(PerturbLaunch p)
+// The FP64 pass over the pixels the FP32 pass listed.  A lane runs its pixel
+// kListChunk iterations at a time and takes the list's next one once
+// kListRefill lanes are idle (counts differ by thousands of iterations from
+// pixel to pixel); chunks of a multiple of four iterations keep the lanes'
+// every-fourth-iteration checks together.  Bound by the FP64 pipe: twelve
+// DFMAs an iteration, 70-77% busy (640x480 at 2^-100 to depth 15000, 1.0e9
+// iterations: 93-118 ms with 30 FP64 instructions an iteration and whole tiles,
+// 42.4 ms now; with 4 blocks of 4 warps an SM, 46.3 with 3, 44.7 with 2, 56
+// with 1).
+constexpr int kListChunk = 64;
+constexpr int kListRefill = 6;
+constexpr int kListBlock = 128;
+constexpr int kListBlocksPerSm = 4;
+
+template <bool WANT_MAG, int FR, bool JU>
+__device__ __forceinline__ void list_pixels(const PerturbLaunch& p)
 {
-    pixel_tiles<T, WANT_MAG, LIST, false, FR, JU>(p);
+    __shared__ unsigned listed[kListBlock / 32][32];   // the warp's current 32 entries
+    // folded formulas: pixels to iterate directly.  They wait here until there
+    // are 32, while their lanes go on with the list: run at once, each lane's
+    // thousands of direct iterations would hold up the other 31.
+    constexpr bool kDirect = FR != MDZ_MANDELBROT;
+    __shared__ DirectPixel direct[kDirect ? kListBlock / 32 : 1][kDirect ? 64 : 1];
+    int nd = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned list_n = *p.list_in_count;
+    const unsigned total = (list_n + 31u) / 32u;
+    unsigned long long its = 0, reb = 0;
+    TileFeed feed;
+    bool active = false;
+    unsigned pix = 0;
+    PixRun<double> r;
+    double dcm_r = 0.0, dcm_i = 0.0;
+    for (;;) {
+        bool fresh = false;
+        feed_lanes(
+            feed, !active,
+            [&]() {
+                const unsigned n = next_tile(feed, &p.sync->tile_counter, p.stop);
+                return n < p.tile_limit && p.tile_base + n < total ? p.tile_base + n : ~0u;
+            },
+            [&](unsigned t, int& px, int&) {
+                px = (int)(t * 32u) + lane;
+                return (unsigned)px < list_n;
+            },
+            [&](int k, int px, int) { listed[warp][k] = p.list_in[px]; },
+            [&](int k) {
+                pix = listed[warp][k];
+                fresh = true;
+            });
+        if (fresh) {
+            const int lrow = (int)(pix / (unsigned)p.W);
+            const int ix = (int)(pix - (unsigned)lrow * (unsigned)p.W);
+            // dc = ((2 ix - W) hs, (H - 2 line) hs), hs = half pixel spacing
+            dcm_r = (double)(2 * ix - p.W) * p.hs_m;
+            dcm_i = (double)(p.H - 2 * (p.row0 + lrow)) * p.hs_m;
+            pixel_start(r, dcm_r, dcm_i, p.hs_e, fold_ke<double>(p));
+            if (JU) {
+                // Julia: the offset is the first delta, at V_0; no dc in the steps
+                r.m = 0;
+                dcm_r = dcm_i = 0.0;
+                refresh_scale(r.st, 0.0, 0.0, p.hs_e);
+            }
+            active = true;
+        }
+        const bool any = __any_sync(0xffffffffu, active);
+        if constexpr (kDirect) {
+            while (nd >= 32 || (!any && nd > 0)) {
+                __syncwarp();
+                const int from = max(nd - 32, 0);
+                if (lane < nd - from) {
+                    const DirectPixel q = direct[warp][from + lane];
+                    float mg = 0.f;
+                    const uint32_t n = fold_direct<FR>(q, p.depth, mg);
+                    p.out[q.pix] = (int32_t)n;
+                    if (WANT_MAG)
+                        p.mag[q.pix] = mg;
+                    its += n ? n : p.depth;
+                }
+                nd = from;
+                __syncwarp();
+            }
+        }
+        if (!any)
+            break;
+        const int enough = (feed.left || feed.more) ? kListRefill : 32;
+        do {
+            uint32_t n = 0;
+            int done = 0;
+            if (active)
+                done = perturb_run<double, kOrbitComplete, FR, JU>(
+                    p, r, dcm_r, dcm_i, p.hs_e, r.wz + (kListChunk - 1), n, nullptr);
+            if (done) {
+                active = false;
+                reb += r.rebases;
+            }
+            if (done == 1) {
+                p.out[pix] = (int32_t)n;
+                if (WANT_MAG)
+                    p.mag[pix] = r.mag;
+                if (r.lost > p.lost_limit && p.flag_out)
+                    p.flag_out[atomicAdd(p.flag_out_count, 1u)] = pix;
+                else
+                    its += n ? n : p.depth;
+            }
+            if constexpr (kDirect) {
+                const unsigned dm = __ballot_sync(0xffffffffu, done == 2);
+                if (done == 2) {
+                    // c = Z_1 + dc
+                    DirectPixel& q = direct[warp][nd + __popc(dm & ((1u << lane) - 1u))];
+                    q.xr = fp_from(r.st.tr);
+                    q.xi = fp_from(r.st.ti);
+                    q.cr = fp_from(ldexp(p.zd[1].x, p.ze[1]) + ldexp(dcm_r, p.hs_e));
+                    q.ci = fp_from(ldexp(p.zd[1].y, p.ze[1]) + ldexp(dcm_i, p.hs_e));
+                    q.wz = r.wz;
+                    q.pix = pix;
+                }
+                nd += __popc(dm);
+                if (nd >= 32)
+                    break;
+            }
+        } while (__popc(__ballot_sync(0xffffffffu, !active)) < enough);
+    }
+    its = warp_sum_u64(its);
+    reb = warp_sum_u64(reb);
+    if (lane == 0) {
+        atomicAdd(&p.sync->iter_sum, its);
+        if (reb)
+            atomicAdd(p.rebases, reb);
+    }
+}
+
+template <class T, bool WANT_MAG, bool LIST, int FR, bool JU>
+__global__ void __launch_bounds__(LIST ? kListBlock : 256) perturb_kernel(PerturbLaunch p)
+{
+    if constexpr (LIST)
+        list_pixels<WANT_MAG, FR, JU>(p);
+    else
+        pixel_tiles<T, WANT_MAG, false, FR, JU>(p);
     if (p.done.count) {
         const unsigned long long total = LIST ? (*p.list_in_count + 31u) / 32u : 0u;
         done_signal(p.done,
@@ -2100,7 +2427,7 @@ __global__ void __launch_bounds__(256, 5) perturb_fused_kernel(OrbitLaunch o, Pe
     __syncthreads();
     if (s_leave)
         return;
-    pixel_tiles<float, WANT_MAG, false, true, MDZ_MANDELBROT>(p);
+    pixel_tiles<float, WANT_MAG, true, MDZ_MANDELBROT>(p);
 }
 
 // ---- serving: one step of the FP32 pass over a mixed work queue ----
@@ -2530,7 +2857,7 @@ int pass_blocks_per_sm(int* out)
     if (!bps) {
         int b = 0;
         MDZ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &b, perturb_kernel<T, WANT_MAG, LIST, FR, JU>, 256, 0));
+            &b, perturb_kernel<T, WANT_MAG, LIST, FR, JU>, LIST ? kListBlock : 256, 0));
         bps = b < 1 ? 1 : b;
     }
     *out = bps;
@@ -2543,13 +2870,16 @@ int launch_pass_fr(mdzgpu_ctx* ctx, const PerturbLaunch& p, cudaStream_t s, long
     int bps = 1;
     if (int rc = pass_blocks_per_sm<T, WANT_MAG, LIST, FR, JU>(&bps))
         return rc;
+    if (LIST && bps > kListBlocksPerSm)
+        bps = kListBlocksPerSm;
     long grid = (long)ctx->num_sms * bps;
-    const long blocks_needed = (work_items + 7) / 8;
+    const int threads = LIST ? kListBlock : 256;
+    const long blocks_needed = (work_items + threads / 32 - 1) / (threads / 32);
     if (grid > blocks_needed)
         grid = blocks_needed;
     if (grid < 1)
         grid = 1;
-    perturb_kernel<T, WANT_MAG, LIST, FR, JU><<<(unsigned)grid, 256, 0, s>>>(p);
+    perturb_kernel<T, WANT_MAG, LIST, FR, JU><<<(unsigned)grid, threads, 0, s>>>(p);
     MDZ_CUDA_TRY(cudaGetLastError());
     return MDZGPU_OK;
 }

@@ -18,8 +18,25 @@ constexpr int kTileH = 4;
 // The warp's current tile: `count` pixels, `left` of them not taken yet.
 struct TileFeed {
     int count = 0, left = 0;
-    bool more = true;   // tiles may be left
+    bool more = true;    // tiles may be left
+    bool first = true;   // no tile pulled yet
 };
+
+// Number of the warp's next tile (on every lane), or ~0u when stopped.  The
+// first one is dealt out, block by block and then warp by warp, so that a
+// launch of few tiles spreads over the SMs and their schedulers (pulled from
+// the counter, the 41 tiles of a list went to the warps of a few SMs: 26 to
+// 33 ms where 41 SMs take 12); later ones come from the counter.
+__device__ __forceinline__ unsigned next_tile(TileFeed& f, unsigned* counter, volatile int* stop)
+{
+    unsigned t = ~0u;
+    const unsigned warps = blockDim.x >> 5;
+    if ((threadIdx.x & 31) == 0 && !(stop && *stop))
+        t = f.first ? (threadIdx.x >> 5) * gridDim.x + blockIdx.x
+                    : warps * gridDim.x + atomicAdd(counter, 1u);
+    f.first = false;
+    return __shfl_sync(0xffffffffu, t, 0);
+}
 
 // Gives pixels to the lanes with `idle` set.  next() returns, on every lane,
 // the next tile's number or ~0u; pixel(tile, px, row) sets the lane's pixel of
