@@ -821,6 +821,7 @@ static int perturb_common(mdzgpu_ctx* ctx, const mdzgpu_frame* f, const mdzgpu_m
             o.fold_parity = 1;
             oq.fold_parity = 0;
         }
+        oq.digits = o.digits + 2 * (size_t)L * q0;   // both are produced at once
         oq.zq = o.zq + q0;
         oq.zd = o.zd + q0;
         oq.ze = o.ze + q0;
@@ -867,8 +868,7 @@ static int perturb_common(mdzgpu_ctx* ctx, const mdzgpu_frame* f, const mdzgpu_m
         MDZ_CUDA_TRY(cudaEventRecord(evo, ctx->side));      // orbit complete
     } else {
         if (!fused) {
-            if ((rc = launch_orbit(o, ctx->stream))
-                || (two && (rc = launch_orbit(oq, ctx->stream)))) {
+            if ((rc = launch_orbit(o, ctx->stream, two ? &oq : nullptr))) {
                 cudaEventDestroy(evo);
                 return rc;
             }

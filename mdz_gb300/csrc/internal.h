@@ -222,7 +222,8 @@ struct OrbitLaunch {
     // gives up (sets progress[4])
     int spin_limit = kSpinLimit;
 };
-int launch_orbit(const OrbitLaunch& p, cudaStream_t s);
+// The orbit, or two orbits of one digit count side by side.
+int launch_orbit(const OrbitLaunch& p, cudaStream_t s, const OrbitLaunch* second = nullptr);
 int orbit_max_limbs();
 
 struct PerturbLaunch {

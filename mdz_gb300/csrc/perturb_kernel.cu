@@ -70,19 +70,22 @@ __device__ __forceinline__ void digit_split(long long v, long long& digit, long 
 
 // value of the 4 digits below the top nonzero one as a double mantissa m and
 // exponent x: value ~ m * 2^x, |m| in [0.5, 1) unless zero.  `scale` is the
-// binary weight of digit 0.
-__device__ void digits_to_double(const int* d, int n, int scale, double& m, int& x)
+// binary weight of digit 0, d(j) digit j of n.
+template <class Digit>
+__device__ __forceinline__ void digits_to_double(const Digit& d, int n, int scale, double& m,
+                                                 int& x)
 {
     int top = n - 1;
-    while (top > 0 && d[top] == 0)
-        --top;
-    double v = (double)d[top];
+    int dt = d(top);
+    while (top > 0 && dt == 0)
+        dt = d(--top);
+    double v = (double)dt;
     if (top >= 1)
-        v += ldexp((double)d[top - 1], -28);
+        v += ldexp((double)d(top - 1), -28);
     if (top >= 2)
-        v += ldexp((double)d[top - 2], -56);
+        v += ldexp((double)d(top - 2), -56);
     if (top >= 3)
-        v += ldexp((double)d[top - 3], -84);
+        v += ldexp((double)d(top - 3), -84);
     int ex = 0;
     m = frexp(v, &ex);
     x = ex + 28 * top + scale;
@@ -358,209 +361,245 @@ __device__ __forceinline__ void orbit_produce(const OrbitLaunch& p, const OrbitP
     }
 }
 
-// The producer of the standalone orbit kernels (orbit_kernel,
-// orbit_stream_kernel), with every thread's work fixed before the loop.
-// Same column sums and carries as orbit_produce, so the same digits; laid
-// out for the shortest serial step: the kept columns are split into
-// kOrbitLeanSlices term slices, and thread q < slices x columns owns one
-// (slice, column) item whose at most MAXP digit pairs are known before the
-// first step (shared-memory indices, padded with a zero entry, so every
-// thread runs the same straight-line code); warps 0 and 1 then add the
-// slices' partial sums of their columns (NSLOT per lane), add C, fold and
-// resolve the carries as orbit_produce does.  The generic loop spent most
-// of its serial step on per-step index arithmetic (divisions, variable trip
-// counts); orbit_produce stays for the fused launch, whose blocks are
-// smaller than slices x columns.
-constexpr int kOrbitLeanSlices = 8;
+// The producer of the standalone orbit kernels (orbit_kernel_lean,
+// orbit_stream_kernel), laid out for the shortest serial step; the same
+// column sums and carries as orbit_produce, so the same digits.  (orbit_produce
+// stays for the fused launch.)
+//
+// What bounds it is latency: nothing of step k + 1 can start before the digits
+// of step k are in shared memory.  A step has one barrier between ceil((L + 2)
+// / 14) warps (none but a warp's own for L <= 12).  A warp owns 16 columns, two
+// lanes each, which halve the column's digit pairs i < j; the first two columns
+// repeat the last two of the warp below, so every carry comes from the same
+// warp.  A pair takes three multiply-adds instead of four: with u = x + y,
+//     A = sum x_i x_j,  B = sum y_i y_j,  S = sum u_i u_j:
+//     Re = A - B,  Im = S - A - B
+// (exact integers; |u| < 2^28 + 2^6, so 40 doubled pairs stay below 2^63).
+// The column's two lanes then swap halves: the even one adds up and carries
+// Re, the odd one Im.  Off the chain of dependent instructions: C enters the
+// sums' start values, doubled digits come from a second copy of Z, Z is
+// double-buffered, the escape test reads the top digits beside the products,
+// and a step's digits go to HBM during the next one.  Cycles a step (before:
+// eight slices a column over 11 warps, partial sums through shared memory and
+// a second barrier to two carry warps): L = 7 332 (1000), 14 486, 26 455, 40
+// 569 (1240 to 1380), 80 1215; burning ship at L = 14 718, celtic 905.
+//
+// The celtic folds need the sign of the whole carried Re^2 - Im^2 before C is
+// added: they exchange the digits through shared memory and carry again.
+constexpr int kOrbitWarpCols = 14;   // columns a warp finishes
 
-template <int MAXP, int NSLOT>
+__host__ __device__ constexpr int orbit_warps(int L)
+{
+    return (L + 2 + kOrbitWarpCols - 1) / kOrbitWarpCols;
+}
+
+// The low 28 bits as a digit in [-2^27, 2^27).
+__device__ __forceinline__ int low_digit(unsigned v)
+{
+    return (int)(v << 4) >> 4;
+}
+
+// The digit of this lane's column after orbit_produce's two carry passes,
+// columns two lanes apart.  With v = d + c 2^28 and the carry cut again, c = e
+// + f 2^28, the first pass leaves t + f' 2^28 (t = d + e', primes: the column
+// below), so the second needs only d, e of the column below and e, f of the
+// one below that: one round of shuffles.  A warp's lowest two columns get no
+// right digits (they are the warp below's; warp 0's lowest is zero).
+__device__ __forceinline__ int carried_digit(long long v)
+{
+    const int d = low_digit((unsigned)v);
+    const long long w = v + (1ll << 27);
+    const int e = low_digit((unsigned)(w >> 28));
+    const int f = ((int)(w >> 32) + (1 << 23)) >> 24;
+    const int e1 = __shfl_up_sync(0xffffffffu, e, 2);
+    const int d1 = __shfl_up_sync(0xffffffffu, d, 2);
+    const int e2 = __shfl_up_sync(0xffffffffu, e, 4);
+    const int f2 = __shfl_up_sync(0xffffffffu, f, 4);
+    return low_digit((unsigned)(d + e1)) + ((d1 + e2 + (1 << 27)) >> 28) + f2;
+}
+
+// Sign of one part of Z (digits at d[0], d[2], ..): the top two digits decide
+// unless both are zero.
+__device__ __forceinline__ int part_sign(const int2* z, int L, bool imag)
+{
+    const int t1 = imag ? z[L - 1].y : z[L - 1].x, t2 = imag ? z[L - 2].y : z[L - 2].x;
+    const int t = t1 ? t1 : t2;
+    if (t)
+        return t > 0 ? 1 : -1;
+    return digits_sign_warp(z, L, imag);
+}
+
+// FOLDS: burning ship, celtic and the variant (else Mandelbrot).
+template <int MAXP, bool FOLDS>
 __device__ __forceinline__ void orbit_produce_lean(const OrbitLaunch& p, const OrbitProgress* prog)
 {
-    constexpr int S = kOrbitLeanSlices;
-    __shared__ int2 z[kMaxOrbitLimbs + 1];                  // z[L] stays zero
-    __shared__ int cc[2][kMaxOrbitLimbs];
-    __shared__ long long part[2][S][kMaxOrbitLimbs + 3];
-    __shared__ float esc[2][2];
-    __shared__ int sgn[2][2];
+    __shared__ int2 zs[2][2][kMaxOrbitLimbs + 1];   // [buffer][Z, 2 Z]; entry L stays zero
+    __shared__ int fold[kMaxOrbitLimbs + 3];        // carried digits of Re^2 - Im^2
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int L = p.limbs;
-    const int P = L + 3;
-    const int cbase = L - 4;
+    const int P = L + 3;           // kept columns L-4 .. 2L-2
+    const int nw = orbit_warps(L);
     const bool from_z0 = p.z0_re != nullptr;
-    const bool ship = p.fractal == MDZ_BURNING_SHIP;
-    const bool celtic = p.fractal == MDZ_GENERALIZED_CELTIC;
-    const bool variant = p.fractal == MDZ_VARIANT;
+    const bool ship = FOLDS && p.fractal == MDZ_BURNING_SHIP;
+    const bool celtic = FOLDS && p.fractal == MDZ_GENERALIZED_CELTIC;
+    const bool variant = FOLDS && p.fractal == MDZ_VARIANT;
     for (int j = threadIdx.x; j < L; j += blockDim.x) {
-        cc[0][j] = p.c_re[j];
-        cc[1][j] = p.c_im[j];
-        if (from_z0) {
-            z[j] = make_int2(p.z0_re[j], p.z0_im[j]);
-            p.digits[j] = p.z0_re[j];
-            p.digits[L + j] = p.z0_im[j];
-        } else {
-            z[j] = make_int2(p.c_re[j], p.c_im[j]);
-            p.digits[j] = 0;                    // Z_0 = 0
+        const int2 z = from_z0 ? make_int2(p.z0_re[j], p.z0_im[j])
+                               : make_int2(p.c_re[j], p.c_im[j]);
+        zs[0][0][j] = z;
+        zs[0][1][j] = make_int2(2 * z.x, 2 * z.y);
+        if (!from_z0) {
+            p.digits[j] = 0;       // Z_0 = 0, Z_1 = C
             p.digits[L + j] = 0;
-            p.digits[2 * L + j] = p.c_re[j];    // Z_1 = C
-            p.digits[3 * L + j] = p.c_im[j];
         }
     }
-    if (threadIdx.x == 0)
-        z[L] = make_int2(0, 0);
-    // this thread's item and its pair indices
-    const int q = threadIdx.x;
-    const bool worker = q < S * P;
-    const int s = worker ? q / P : 0;
-    const int pos = worker ? q - s * P : 0;
-    const int c = cbase + pos;
+    if (threadIdx.x < 4)
+        zs[threadIdx.x >> 1][threadIdx.x & 1][L] = make_int2(0, 0);
+    // this lane's column, half and (after the swap) part; its pairs' places
+    const int half = lane & 1, part = half;
+    const int g = lane >> 1;
+    const int pos = kOrbitWarpCols * warp + g - 1;
+    const bool column = warp < nw && pos >= 0 && pos < P;
+    const bool owner = column && g >= 2 && pos >= 3;
+    const int c = L - 4 + pos;
     const int lo = c - (L - 1) > 0 ? c - (L - 1) : 0;
     const int hi = (c - 1) >> 1;
     int ia[MAXP], ib[MAXP];
 #pragma unroll
     for (int j = 0; j < MAXP; ++j) {
-        const int i = lo + s + S * j;
-        const bool ok = worker && i <= hi;
+        const int i = lo + half + 2 * j;
+        const bool ok = column && i <= hi;
         ia[j] = ok ? i : L;
         ib[j] = ok ? c - i : L;
     }
-    const int ih = (worker && s == 0 && !(c & 1)) ? (c >> 1) : L;
+    const int ih = (column && half == 0 && !(c & 1)) ? (c >> 1) : L;
+    const bool has_c = column && pos >= 3;
+    const long long cre = has_c ? p.c_re[pos - 3] : 0, cim = has_c ? p.c_im[pos - 3] : 0;
+    const long long cc = part ? cim : cre;
+    // C in the sums' start: Re = A - B, Im = S - A - B
+    const long long A0 = !FOLDS && half == 0 ? cre : 0, S0 = !FOLDS && half == 0 ? cim + cre : 0;
+    int k = from_z0 ? 0 : 1;
+    // this lane's digit of Z_k, stored one step late
+    int d = 0;
+    if (owner)
+        d = from_z0 ? (part ? p.z0_im[pos - 3] : p.z0_re[pos - 3]) : (int)cc;
+    int* out = p.digits + (size_t)k * 2 * L + (owner ? part * L + pos - 3 : 0);
     __threadfence();
     __syncthreads();
-    int k = from_z0 ? 0 : 1;
-    // top-digit estimate (escape test) and, for burning ship, the sign of
-    // part pt of the Z just written (all lanes of warp pt)
-    auto summary = [&](int pt, int slot) {
-        __syncwarp();
-        if (lane == 0) {
-            const int2 t1 = z[L - 1], t2 = z[L - 2];
-            esc[pt][slot] = pt ? fmaf((float)t2.y, 3.7252903e-9f, (float)t1.y)
-                               : fmaf((float)t2.x, 3.7252903e-9f, (float)t1.x);
-        }
-        if (ship) {
-            const int sg = digits_sign_warp(z, L, pt == 1);
-            if (lane == 0)
-                sgn[pt][slot] = sg;
-        }
+    auto barrier = [&]() {
+        if (nw == 1)
+            __syncwarp();
+        else
+            asm volatile("bar.sync 1, %0;" ::"r"(32 * nw) : "memory");
     };
-    if (warp < 2)
-        summary(warp, k & 1);
-    for (;; ++k) {
-        __syncthreads();  // A: Z_k, its estimate and signs complete
+    // Z_k in zk -> Z_{k+1} in zn; false when Z_k escaped or was the last
+    auto step = [&](const int2 (&zk)[2][kMaxOrbitLimbs + 1],
+                    int2 (&zn)[2][kMaxOrbitLimbs + 1]) -> bool {
+        barrier();   // Z_k complete; Z_{k-1} no longer read
         if (prog && (k & 63) == 0 && threadIdx.x == 0)
-            *(volatile int*)prog->raw_len = k + 1;
-        if (worker) {
-            long long r0 = 0, r1 = 0, m0 = 0, m1 = 0;
+            *(volatile int*)prog->raw_len = k;   // fenced at the last step's end
+        long long A, B, S;
+        {
+            const int2 h = zk[0][ih];
+            A = A0 + (long long)h.x * h.x;
+            B = (long long)h.y * h.y;
+            S = S0 + (long long)(h.x + h.y) * (h.x + h.y);
+        }
+        if constexpr (MAXP < 10) {
 #pragma unroll
             for (int j = 0; j < MAXP; ++j) {
-                const int2 a = z[ia[j]], b = z[ib[j]];
-                if (j & 1) {
-                    r1 += (long long)a.x * b.x;
-                    r1 -= (long long)a.y * b.y;
-                    m1 += (long long)a.x * b.y;
-                    m1 += (long long)b.x * a.y;
-                } else {
-                    r0 += (long long)a.x * b.x;
-                    r0 -= (long long)a.y * b.y;
-                    m0 += (long long)a.x * b.y;
-                    m0 += (long long)b.x * a.y;
+                const int2 a = zk[0][ia[j]], b = zk[1][ib[j]];
+                A += (long long)a.x * b.x;
+                B += (long long)a.y * b.y;
+                S += (long long)(a.x + a.y) * (b.x + b.y);
+            }
+        } else {
+            // all loads first, two sums a column each: L = 40 takes 569 cycles
+            // a step, 642 the other way, L = 80 the same both ways; L = 26
+            // 525 and 455
+            const unsigned za = (unsigned)__cvta_generic_to_shared(&zk[0][0]);
+            const unsigned zb = (unsigned)__cvta_generic_to_shared(&zk[1][0]);
+            int2 a[MAXP], b[MAXP];
+            long long A1 = 0, B1 = 0, S1 = 0;
+#pragma unroll
+            for (int j = 0; j < MAXP; ++j) {
+                asm volatile("ld.shared.v2.s32 {%0, %1}, [%2];"
+                             : "=r"(a[j].x), "=r"(a[j].y) : "r"(za + 8 * ia[j]) : "memory");
+                asm volatile("ld.shared.v2.s32 {%0, %1}, [%2];"
+                             : "=r"(b[j].x), "=r"(b[j].y) : "r"(zb + 8 * ib[j]) : "memory");
+            }
+#pragma unroll
+            for (int j = 0; j < MAXP; ++j) {
+                (j & 1 ? A1 : A) += (long long)a[j].x * b[j].x;
+                (j & 1 ? B1 : B) += (long long)a[j].y * b[j].y;
+                (j & 1 ? S1 : S) += (long long)(a[j].x + a[j].y) * (b[j].x + b[j].y);
+            }
+            A += A1;
+            B += B1;
+            S += S1;
+        }
+        if (owner)
+            *out = d;
+        out += 2 * L;
+        const int2 t1 = zk[0][L - 1], t2 = zk[0][L - 2];
+        const long long re = A - B, im = S - A - B;
+        // the halves of the part this lane finishes
+        long long v = (part ? im : re) + __shfl_xor_sync(0xffffffffu, part ? re : im, 1);
+        if (ship) {
+            // Im' = 2 |Re| |Im| + Ci = sign(Re) sign(Im) 2 Re Im + Ci
+            const int sxy = part_sign(zk[0], L, false) * part_sign(zk[0], L, true);
+            if (part)
+                v = sxy < 0 ? -v : (sxy > 0 ? v : 0);
+        }
+        if (celtic || (variant && (k & 1) == p.fold_parity)) {
+            // Re' = |Re^2 - Im^2| + Cr: the sign is that of the carried
+            // digits' most significant nonzero one
+            const bool re_part = part == 0;
+            d = carried_digit(re_part ? v : v + cc);
+            if (re_part && column && (g >= 2 || warp == 0))
+                fold[pos] = d;
+            barrier();
+            const int top = fold[P - 1] ? fold[P - 1] : fold[P - 2];
+            bool neg = top < 0;
+            if (!top) {
+                int sg = 0;
+#pragma unroll
+                for (int t = 2; t >= 0; --t) {
+                    const int q = lane + 32 * t;
+                    const int f = q < P ? fold[q] : 0;
+                    const unsigned m = __ballot_sync(0xffffffffu, f != 0);
+                    const int x = __shfl_sync(0xffffffffu, f, m ? 31 - __clz(m) : 0);
+                    if (m && !sg)
+                        sg = x > 0 ? 1 : -1;
                 }
+                neg = sg < 0;
             }
-            const int2 h = z[ih];
-            long long re = 2 * (r0 + r1), im = 2 * (m0 + m1);
-            re += (long long)h.x * h.x;
-            re -= (long long)h.y * h.y;
-            im += 2 * ((long long)h.x * h.y);
-            part[0][s][pos] = re;
-            part[1][s][pos] = im;
+            const int w = (re_part && column) ? (neg ? -fold[pos] : fold[pos]) : 0;
+            const int dr = carried_digit(re_part ? w + cc : 0);
+            if (re_part)
+                d = dr;
+        } else {
+            d = carried_digit(FOLDS ? v + cc : v);
         }
-        const float ea = esc[0][k & 1], eb = esc[1][k & 1];
-        const bool stop = fmaf(ea, ea, eb * eb) > 4.0f || k >= p.max_k;
-        const int sxy = ship ? sgn[0][k & 1] * sgn[1][k & 1] : 1;
-        __syncthreads();  // B: partial sums in place; every read of Z_k done
-        if (stop)
-            break;
-        if (warp >= 2)
-            continue;
-        // Z_{k+1}: warp 0 the real part, warp 1 the imaginary part
-        const int pt = warp;
-        const bool fold_re = pt == 0 && (celtic || (variant && (k & 1) == p.fold_parity));
-        long long v[NSLOT];
-#pragma unroll
-        for (int t = 0; t < NSLOT; ++t) {
-            const int pp = lane + 32 * t;
-            long long a = 0;
-            if (pp < P) {
-                long long u[S];
-#pragma unroll
-                for (int ss = 0; ss < S; ++ss)
-                    u[ss] = part[pt][ss][pp];
-                a = ((u[0] + u[1]) + (u[2] + u[3])) + ((u[4] + u[5]) + (u[6] + u[7]));
-                if (pt == 1)
-                    a *= sxy;
-                if (pp >= 3 && !fold_re)
-                    a += cc[pt][pp - 3];
-            }
-            v[t] = a;
+        if (owner) {
+            (part ? zn[0][pos - 3].y : zn[0][pos - 3].x) = d;
+            (part ? zn[1][pos - 3].y : zn[1][pos - 3].x) = 2 * d;
         }
-        auto carry2 = [&]() {
-#pragma unroll
-            for (int pass = 0; pass < 2; ++pass) {
-                long long dg[NSLOT], cy[NSLOT];
-#pragma unroll
-                for (int t = 0; t < NSLOT; ++t)
-                    digit_split(v[t], dg[t], cy[t]);
-#pragma unroll
-                for (int t = 0; t < NSLOT; ++t) {
-                    long long in = __shfl_up_sync(0xffffffffu, cy[t], 1);
-                    const long long wrap =
-                        __shfl_sync(0xffffffffu, t > 0 ? cy[t - 1] : 0ll, 31);
-                    if (lane == 0)
-                        in = wrap;
-                    v[t] = dg[t] + in;
-                }
-            }
-        };
-        carry2();
-        if (fold_re) {
-            int sg = 0;
-#pragma unroll
-            for (int t = NSLOT - 1; t >= 0; --t) {
-                const int pp = lane + 32 * t;
-                const bool ok = pp < P && v[t] != 0;
-                const unsigned m = __ballot_sync(0xffffffffu, ok);
-                if (m && !sg) {
-                    const long long x = __shfl_sync(0xffffffffu, v[t], 31 - __clz(m));
-                    sg = x > 0 ? 1 : -1;
-                }
-            }
-#pragma unroll
-            for (int t = 0; t < NSLOT; ++t) {
-                const int pp = lane + 32 * t;
-                if (sg < 0)
-                    v[t] = -v[t];
-                if (pp < P && pp >= 3)
-                    v[t] += cc[0][pp - 3];
-            }
-            carry2();
+        // top-digit estimate of |Z_k|^2; nothing of a step past an escape
+        // leaves the block
+        const float ea = fmaf((float)t2.x, 3.7252903e-9f, (float)t1.x);
+        const float eb = fmaf((float)t2.y, 3.7252903e-9f, (float)t1.y);
+        if (fmaf(ea, ea, eb * eb) > 4.0f || k >= p.max_k)
+            return false;
+        ++k;
+        if (prog && (k & 63) == 0)
+            __threadfence();  // the digits of Z_{k-1} before raw_len = k
+        return true;
+    };
+    if (warp < nw)
+        while (step(zs[0], zs[1]) && step(zs[1], zs[0])) {
         }
-        int* out = p.digits + (size_t)(k + 1) * 2 * L + pt * L;
-#pragma unroll
-        for (int t = 0; t < NSLOT; ++t) {
-            const int pp = lane + 32 * t;
-            if (pp >= 3 && pp < P) {
-                const int d = (int)v[t];
-                if (pt == 0)
-                    z[pp - 3].x = d;
-                else
-                    z[pp - 3].y = d;
-                out[pp - 3] = d;
-            }
-        }
-        summary(pt, (k + 1) & 1);
-        if (prog && ((k + 1) & 63) == 0)
-            __threadfence();  // Z_{k+1}'s digits before raw_len = k + 2
-    }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -573,22 +612,23 @@ __device__ __forceinline__ void orbit_produce_lean(const OrbitLaunch& p, const O
     }
 }
 
-// (MAXP, NSLOT) of the lean producer for L digits: a column holds at most
-// floor(L / 2) pairs, spread over 8 slices; L + 3 columns over 32 lanes.
+// (L, MAXP) of the lean producer: a column of L digits holds at most
+// floor(L / 2) pairs, half of them a lane's.
 #define MDZ_ORBIT_LEAN_CASES(X) \
-    X(17, 1, 1) X(29, 2, 1) X(33, 2, 2) X(49, 3, 2) X(61, 4, 2) X(65, 4, 3) X(80, 5, 3)
+    X(9, 2) X(13, 3) X(21, 5) X(29, 7) X(41, 10) X(53, 13) X(65, 16) X(80, 20)
 
-// Threads of a lean launch: slices x columns, rounded to 512 or 1024 (the
-// finisher of the streamed orbit works in batches of its block size, which
-// must divide 1024).
-__host__ __device__ constexpr int orbit_lean_threads(int L)
-{
-    return kOrbitLeanSlices * (L + 3) <= 512 ? 512 : 1024;
-}
+// Threads of the streamed orbit's two blocks: the finisher works in batches of
+// its block size, which must divide 1024; the producer needs orbit_warps(L) <=
+// 6 warps of it.
+constexpr int kOrbitStreamThreads = 512;
+static_assert(orbit_warps(kMaxOrbitLimbs) * 32 <= kOrbitStreamThreads, "producer's warps");
 
-template <int MAXP, int NSLOT>
-__global__ void __launch_bounds__(1024) orbit_kernel_lean(OrbitLaunch p)
+// Block b produces orbit b.
+template <int MAXP, bool FOLDS>
+__global__ void __launch_bounds__(orbit_warps(kMaxOrbitLimbs) * 32)
+    orbit_kernel_lean(OrbitLaunch first, OrbitLaunch second)
 {
+    const OrbitLaunch& p = blockIdx.x ? second : first;
     unsigned smid = 0;
     if (p.sm_busy) {
         asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
@@ -596,7 +636,7 @@ __global__ void __launch_bounds__(1024) orbit_kernel_lean(OrbitLaunch p)
         if (threadIdx.x == 0)
             atomicAdd(p.sm_busy + smid, 1);
     }
-    orbit_produce_lean<MAXP, NSLOT>(p, nullptr);
+    orbit_produce_lean<MAXP, FOLDS>(p, nullptr);
     if (p.sm_busy && threadIdx.x == 0)
         atomicSub(p.sm_busy + smid, 1);
 }
@@ -610,14 +650,14 @@ __global__ void __launch_bounds__(1024) orbit_kernel_lean(OrbitLaunch p)
 __device__ __noinline__ void finish_entry(const OrbitLaunch& p, int k, bool from_l2)
 {
     const int L = p.limbs;
-    int dr[kMaxOrbitLimbs], di[kMaxOrbitLimbs];
     const int* src = p.digits + (size_t)k * 2 * L;
-    for (int j = 0; j < L; ++j) {
-        // in the fused launch the digits were written by another block while
-        // this one runs: read them from L2, never from a stale L1 line
-        dr[j] = from_l2 ? __ldcg(src + j) : src[j];
-        di[j] = from_l2 ? __ldcg(src + L + j) : src[L + j];
-    }
+    // Digits as they are needed: the top few, unless all of them are (a copy of
+    // all into local memory, as before, made the streamed orbit's finisher the
+    // slower of its two blocks: 89 ms for 200 002 entries of 40 digits).
+    // Streamed digits are written by another block while this one runs: they
+    // are read from L2, never from a stale L1 line.
+    auto dr = [&](int j) { return from_l2 ? __ldcg(src + j) : src[j]; };
+    auto di = [&](int j) { return from_l2 ? __ldcg(src + L + j) : src[L + j]; };
     const int F = 28 * (L - 1);
     double mr, mi;
     int xr, xi;
@@ -652,10 +692,11 @@ __device__ __noinline__ void finish_entry(const OrbitLaunch& p, int k, bool from
             long long cd = 0, cs = 0;
             for (int j = 0; j < L; ++j) {
                 long long d, cy;
-                digit_split(sr * (long long)dr[j] - si * (long long)di[j] + cd, d, cy);
+                const int x = dr(j), y = di(j);
+                digit_split(sr * (long long)x - si * (long long)y + cd, d, cy);
                 dd[j] = (int)d;
                 cd = cy;
-                digit_split(sr * (long long)dr[j] + si * (long long)di[j] + cs, d, cy);
+                digit_split(sr * (long long)x + si * (long long)y + cs, d, cy);
                 ss[j] = (int)d;
                 cs = cy;
             }
@@ -664,8 +705,8 @@ __device__ __noinline__ void finish_entry(const OrbitLaunch& p, int k, bool from
             ss[L - 1] += (int)(cs << 28);
             double md, ms;
             int xd, xs;
-            digits_to_double(dd, L, -F, md, xd);
-            digits_to_double(ss, L, -F, ms, xs);
+            digits_to_double([&](int j) { return dd[j]; }, L, -F, md, xd);
+            digits_to_double([&](int j) { return ss[j]; }, L, -F, ms, xs);
             fmv = md * ms;
             fev = xd + xs;
         }
@@ -695,7 +736,7 @@ __device__ __noinline__ void finish_entry(const OrbitLaunch& p, int k, bool from
         const int ilo = c - (L - 1) > 0 ? c - (L - 1) : 0;
         const int ihi = c < L - 1 ? c : L - 1;
         for (int i = ilo; i <= ihi; ++i)
-            acc += (long long)dr[i] * dr[c - i] + (long long)di[i] * di[c - i];
+            acc += (long long)dr(i) * dr(c - i) + (long long)di(i) * di(c - i);
         col[c] = acc;
     }
     col[ncol - 1] -= 4;
@@ -712,7 +753,7 @@ __device__ __noinline__ void finish_entry(const OrbitLaunch& p, int k, bool from
     dig[ncol - 1] += (int)(carry << 28);
     double m;
     int x;
-    digits_to_double(dig, ncol, -2 * F, m, x);
+    digits_to_double([&](int j) { return dig[j]; }, ncol, -2 * F, m, x);
     p.dd[k] = m;
     p.de[k] = x;
 }
@@ -2564,8 +2605,8 @@ __global__ void __launch_bounds__(256, FR == MDZ_MANDELBROT ? 5 : 4)
 // 1: the finisher (batches of blockDim.x entries).  Launched cooperatively
 // (both blocks resident at once: the finisher waits, bounded, on the
 // producer's progress).
-template <int MAXP, int NSLOT>
-__global__ void __launch_bounds__(1024) orbit_stream_kernel(OrbitLaunch o, OrbitProgress g,
+template <int MAXP, bool FOLDS>
+__global__ void __launch_bounds__(kOrbitStreamThreads) orbit_stream_kernel(OrbitLaunch o, OrbitProgress g,
                                                             int* producer_sm, DoneSignal done)
 {
     if (blockIdx.x == 0) {
@@ -2576,7 +2617,7 @@ __global__ void __launch_bounds__(1024) orbit_stream_kernel(OrbitLaunch o, Orbit
                 atomicAdd(o.sm_busy + smid % (unsigned)o.sm_words, 1);
             *(volatile int*)producer_sm = (int)smid + 1;
         }
-        orbit_produce_lean<MAXP, NSLOT>(o, &g);
+        orbit_produce_lean<MAXP, FOLDS>(o, &g);
         if (threadIdx.x == 0) {
             *(volatile int*)producer_sm = 0;
             if (o.sm_busy)
@@ -2781,13 +2822,13 @@ int launch_orbit_stream(const OrbitLaunch& o, int* progress, cudaStream_t s, Don
     int* producer_sm = progress + 5;
     void* args[] = {&oo, &g, &producer_sm, &done};
     const void* fn = nullptr;
-#define MDZ_CASE(lmax, mp, ns)                                      \
+#define MDZ_CASE(lmax, mp)                                          \
     if (!fn && o.limbs <= lmax)                                     \
-        fn = (const void*)orbit_stream_kernel<mp, ns>;
+        fn = o.fractal == MDZ_MANDELBROT ? (const void*)orbit_stream_kernel<mp, false> \
+                                         : (const void*)orbit_stream_kernel<mp, true>;
     MDZ_ORBIT_LEAN_CASES(MDZ_CASE)
 #undef MDZ_CASE
-    MDZ_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(2), dim3(orbit_lean_threads(o.limbs)),
-                                             args, 0, s));
+    MDZ_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(2), dim3(kOrbitStreamThreads), args, 0, s));
     return MDZGPU_OK;
 }
 
@@ -2830,23 +2871,31 @@ int launch_perturb_step(int num_sms, const PerturbLaunch& p, const unsigned* in,
     return MDZGPU_OK;
 }
 
-int launch_orbit(const OrbitLaunch& p, cudaStream_t s)
+int launch_orbit(const OrbitLaunch& p, cudaStream_t s, const OrbitLaunch* second)
 {
     if (p.limbs < 5 || p.limbs > kMaxOrbitLimbs) {
         set_error("orbit: %d limbs outside [5, %d]", p.limbs, kMaxOrbitLimbs);
         return MDZGPU_ERR_UNSUPPORTED;
     }
     bool launched = false;
-#define MDZ_CASE(lmax, mp, ns)                                                   \
-    if (!launched && p.limbs <= lmax) {                                          \
-        orbit_kernel_lean<mp, ns><<<1, orbit_lean_threads(p.limbs), 0, s>>>(p); \
-        launched = true;                                                         \
+    const OrbitLaunch& q = second ? *second : p;
+    const unsigned blocks = second ? 2 : 1;
+#define MDZ_CASE(lmax, mp)                                                             \
+    if (!launched && p.limbs <= lmax) {                                                \
+        if (p.fractal == MDZ_MANDELBROT)                                               \
+            orbit_kernel_lean<mp, false><<<blocks, 32 * orbit_warps(p.limbs), 0, s>>>(p, q); \
+        else                                                                           \
+            orbit_kernel_lean<mp, true><<<blocks, 32 * orbit_warps(p.limbs), 0, s>>>(p, q);  \
+        launched = true;                                                               \
     }
     MDZ_ORBIT_LEAN_CASES(MDZ_CASE)
 #undef MDZ_CASE
     MDZ_CUDA_TRY(cudaGetLastError());
-    orbit_finish_kernel<<<(p.max_k + 1 + 127) / 128, 128, 0, s>>>(p);
-    MDZ_CUDA_TRY(cudaGetLastError());
+    for (unsigned b = 0; b < blocks; ++b) {
+        const OrbitLaunch& o = b ? q : p;
+        orbit_finish_kernel<<<(o.max_k + 1 + 127) / 128, 128, 0, s>>>(o);
+        MDZ_CUDA_TRY(cudaGetLastError());
+    }
     return MDZGPU_OK;
 }
 
@@ -2948,9 +2997,11 @@ int preload_perturb_kernels()
     if (!rc)
         rc = preload_fr<MDZ_GENERALIZED_CELTIC>();
     cudaFuncAttributes a;
-#define MDZ_CASE(lmax, mp, ns)                                                        \
-    if (!rc && (cudaFuncGetAttributes(&a, orbit_stream_kernel<mp, ns>) != cudaSuccess \
-                || cudaFuncGetAttributes(&a, orbit_kernel_lean<mp, ns>) != cudaSuccess)) \
+#define MDZ_CASE(lmax, mp)                                                            \
+    if (!rc && (cudaFuncGetAttributes(&a, orbit_stream_kernel<mp, false>) != cudaSuccess    \
+                || cudaFuncGetAttributes(&a, orbit_stream_kernel<mp, true>) != cudaSuccess  \
+                || cudaFuncGetAttributes(&a, orbit_kernel_lean<mp, false>) != cudaSuccess   \
+                || cudaFuncGetAttributes(&a, orbit_kernel_lean<mp, true>) != cudaSuccess))  \
         rc = MDZGPU_ERR_CUDA;
     MDZ_ORBIT_LEAN_CASES(MDZ_CASE)
 #undef MDZ_CASE
