@@ -293,6 +293,9 @@ int launch_orbit_stream(const OrbitLaunch& o, int* progress, cudaStream_t s,
 // unfinished ones go to out; counters[0] = pull counter, counters[1] = out
 // count, counters[2] = working blocks (all reset by the launch).  Blocks
 // placed on the orbit producer's SM (p.producer_sm) leave it to the producer.
+// Whether a step over n pixels takes two a lane (perturb_pairs_kernel): where
+// the deltas start below the FP32 range and every warp of the chip gets 64.
+bool perturb_in_pairs(int num_sms, const PerturbLaunch& p, size_t n);
 int launch_perturb_step(int num_sms, const PerturbLaunch& p, const unsigned* in, unsigned n,
                         unsigned* out, unsigned* counters, uint4* state, unsigned budget,
                         cudaStream_t s, cudaEvent_t before = nullptr,

@@ -2718,6 +2718,349 @@ __global__ void __launch_bounds__(256, FR == MDZ_MANDELBROT ? 5 : 4)
     }
 }
 
+// ---- two pixels a lane: the deep part of a Mandelbrot frame ----
+
+// Packed pair of floats (pixel a, pixel b); fma.rn.f32x2 rounds each half as
+// fmaf does.
+__device__ __forceinline__ uint64_t pair_of(float a, float b)
+{
+    return ((uint64_t)__float_as_uint(b) << 32) | __float_as_uint(a);
+}
+__device__ __forceinline__ float pair_a(uint64_t v)
+{
+    return __uint_as_float((uint32_t)v);
+}
+__device__ __forceinline__ float pair_b(uint64_t v)
+{
+    return __uint_as_float((uint32_t)(v >> 32));
+}
+__device__ __forceinline__ uint64_t pair_fma(uint64_t x, uint64_t y, uint64_t z)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+    return r;
+}
+
+// Whether a pixel may run in whole blocks with the reference's z (dz below the
+// FP32 range).
+__device__ __forceinline__ bool deep_state(const PixRun<float>& r)
+{
+    return r.st.s == 0.f && !r.st.force_slow;
+}
+
+// |t| outside [2^-32, 2^32] (and not 0)
+__device__ __forceinline__ bool needs_scale(float amax)
+{
+    return (amax > 4.2949673e9f || amax < 2.3283064e-10f) && amax != 0.f;
+}
+
+__device__ __forceinline__ bool pair_rescale(PixRun<float>& r, float dcf_r, float dcf_i, int dce)
+{
+    const float amax = fmaxf(fabsf(r.st.tr), fabsf(r.st.ti));
+    if (!needs_scale(amax))
+        return true;
+    const int k = Mant<float>::exponent_of(amax);
+    const float sc = Mant<float>::scale(1.f, -k);
+    r.st.tr *= sc;
+    r.st.ti *= sc;
+    r.st.e += k;
+    refresh_scale(r.st, dcf_r, dcf_i, dce);
+    return r.st.s == 0.f && !r.st.force_slow;
+}
+
+// 32 orbit entries for a warp: (2x, 2x, 2y, 2y) and (-2y, -2y).
+struct PairStage {
+    float4 xy[32];
+    float2 ny[32];
+};
+
+// N steps t' = 2 Z t + dc 2^-e of two pixels from the staged entries at zp / zn.
+template <int N>
+__device__ __forceinline__ void pair_steps(unsigned zp, unsigned zn, uint64_t& tr, uint64_t& ti,
+                                           uint64_t dcr, uint64_t dci)
+{
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        uint64_t x, y, ny;
+        asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];"
+                     : "=l"(x), "=l"(y) : "r"(zp + 16 * u) : "memory");
+        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(ny) : "r"(zn + 8 * u) : "memory");
+        const uint64_t r = pair_fma(x, tr, pair_fma(ny, ti, dcr));
+        ti = pair_fma(x, ti, pair_fma(y, tr, dci));
+        tr = r;
+    }
+}
+
+// The deep-zoom blocks of perturb_run for the warp's pixel pairs that are at
+// the first such pair's m and wz (`pair`: this lane's two pixels are at one
+// entry and deep_state): whole blocks of four up to iteration `last`, the last
+// finished entry, or an entry that needs attention; the values are those of
+// each pixel alone.  The warp copies 32 orbit entries at a time to shared
+// memory, each component twice, so a step of two pixels is two broadcast loads
+// and four packed FMAs.  (An orbit load from L1 costs an SM about 3.7 cycles a
+// warp, whatever its width: it bounded the loop at one pixel a lane, 3.3 cycles
+// a step of 32 pixels.  A step of 64 takes 4.4 now, 10.5 warp instructions; with
+// the rescale check every four steps 5.2.)  All lanes call it; returns whether
+// this lane's pair took part.
+__device__ __forceinline__ bool deep_pairs(const PerturbLaunch& p, PairStage& stage, bool pair,
+                                           PixRun<float>& a, PixRun<float>& b, uint32_t last,
+                                           int avail, float adcr, float adci, float bdcr,
+                                           float bdci)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned who = __ballot_sync(0xffffffffu, pair);
+    if (!who)
+        return false;
+    int m = __shfl_sync(0xffffffffu, a.m, __ffs(who) - 1);
+    uint32_t wz = __shfl_sync(0xffffffffu, a.wz, __ffs(who) - 1);
+    const bool in = pair && a.m == m && a.wz == wz;
+    last = __reduce_min_sync(0xffffffffu, in ? last : 0xffffffffu);
+    avail = __reduce_min_sync(0xffffffffu, in ? avail : 0x7fffffff);
+    const int mfirst = m;
+    // (lanes not in run along on t = 1, dc = 0, unheeded)
+    uint64_t tr = pair_of(1.f, 1.f), ti = tr, dcr = 0, dci = 0;
+    if (in) {
+        tr = pair_of(a.st.tr, b.st.tr);
+        ti = pair_of(a.st.ti, b.st.ti);
+        dcr = pair_of(a.st.dcr, b.st.dcr);
+        dci = pair_of(a.st.dci, b.st.dci);
+    }
+    bool deep = true;
+    while (deep && wz + 3u <= last && m + 4 < avail && five_clear(p.att, m)) {
+        const int mstart = m;
+        const int span = (int)min(last - wz, 0x3fffffffu);
+        const int mmax = min(span + m - 3, avail - 5);
+        // the clear run of the attention mask, as in perturb_run: 32 words at
+        // once, those that hold finished entries
+        const int word = (m >> 5) + lane;
+        unsigned w = 32 * word < avail ? __ldg(p.att + word) : 1u;
+        if (lane == 0)
+            w &= 0xffffffffu << (m & 31);
+        const unsigned set = __ballot_sync(0xffffffffu, w != 0u);
+        const int at = set ? __ffs(set) - 1 : 0;
+        const unsigned first = __shfl_sync(0xffffffffu, w, at);
+        const int nxt = set ? 32 * ((m >> 5) + at) + __ffs(first) - 1 : 32 * ((m >> 5) + 32);
+        int nb = (min(mmax, nxt - 5) - m) / 4 + 1;   // blocks, at least one
+        float4 ahead = lane < 4 * nb ? p.zq[m + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+        while (deep && nb > 0) {
+            stage.xy[lane] = make_float4(ahead.x, ahead.x, ahead.y, ahead.y);
+            stage.ny[lane] = make_float2(-ahead.y, -ahead.y);
+            __syncwarp();
+            int n8 = min(nb, 8);
+            nb -= n8;
+            if (lane < 4 * nb)
+                ahead = p.zq[m + 32 + lane];
+            m += 4 * n8;
+            unsigned zp = (unsigned)__cvta_generic_to_shared(stage.xy);
+            unsigned zn = (unsigned)__cvta_generic_to_shared(stage.ny);
+            bool coarse = true;
+            while (deep && n8 > 0) {
+                bool out;
+                if (coarse && n8 >= 4) {
+                    // sixteen steps a check: |t| grows by at most 2^2.5 a step
+                    // (and to |dc 2^-e|); where it leaves [2^-90, 2^90] the
+                    // sixteen are redone in fours
+                    uint64_t tr0, ti0;
+                    float ma, mb;
+                    do {
+                        tr0 = tr;
+                        ti0 = ti;
+#pragma unroll 1
+                        for (int h = 0; h < 2; ++h) {
+                            pair_steps<8>(zp, zn, tr, ti, dcr, dci);
+                            zp += 128;
+                            zn += 64;
+                        }
+                        n8 -= 4;
+                        ma = fmaxf(fabsf(pair_a(tr)), fabsf(pair_a(ti)));
+                        mb = fmaxf(fabsf(pair_b(tr)), fabsf(pair_b(ti)));
+                        out = !(fmaxf(ma, mb) <= 4.2949673e9f && fminf(ma, mb) >= 2.3283064e-10f);
+                        out = __any_sync(0xffffffffu, out);
+                    } while (n8 >= 4 && !out);
+                    if (out
+                        && __any_sync(0xffffffffu, in && !(ma < 1.2e27f && (ma > 8e-28f || ma == 0.f)
+                                                           && mb < 1.2e27f
+                                                           && (mb > 8e-28f || mb == 0.f)))) {
+                        tr = tr0;
+                        ti = ti0;
+                        zp -= 256;
+                        zn -= 128;
+                        n8 += 4;
+                        coarse = false;
+                        continue;
+                    }
+                } else {
+                    pair_steps<4>(zp, zn, tr, ti, dcr, dci);
+                    zp += 64;
+                    zn += 32;
+                    --n8;
+                    out = true;
+                }
+                // the rescale check of the general path (a power of two: where
+                // it happens changes no value)
+                if (out && in) {
+                    a.st.tr = pair_a(tr);
+                    a.st.ti = pair_a(ti);
+                    b.st.tr = pair_b(tr);
+                    b.st.ti = pair_b(ti);
+                    const bool da = pair_rescale(a, adcr, adci, p.hs_e);
+                    const bool db = pair_rescale(b, bdcr, bdci, p.hs_e);
+                    deep = da && db;
+                    tr = pair_of(a.st.tr, b.st.tr);
+                    ti = pair_of(a.st.ti, b.st.ti);
+                    dcr = pair_of(a.st.dcr, b.st.dcr);
+                    dci = pair_of(a.st.dci, b.st.dci);
+                }
+                deep = __all_sync(0xffffffffu, deep);
+            }
+            m -= 4 * n8;
+            __syncwarp();
+        }
+        wz += (uint32_t)(m - mstart);
+    }
+    if (in) {
+        a.st.tr = pair_a(tr);
+        a.st.ti = pair_a(ti);
+        b.st.tr = pair_b(tr);
+        b.st.ti = pair_b(ti);
+        a.m = b.m = m;
+        a.wz = b.wz = wz;
+        if (m != mfirst)
+            a.mag = b.mag = p.zq[m].z;
+    }
+    return in;
+}
+
+// perturb_step_kernel for a Mandelbrot frame whose deltas start below the FP32
+// range: a lane takes two pixels and steps them together as long as they are
+// at the same orbit entry (from the frame's start until one of them leaves
+// the deep part or rebases).  What bounds it is issue: 9.5 warp instructions a
+// pixel-iteration one pixel at a time.
+template <bool WANT_MAG>
+__global__ void __launch_bounds__(256, 3) perturb_pairs_kernel(PerturbLaunch p, FrameStep q)
+{
+    __shared__ int s_leave;
+    if (threadIdx.x == 0) {
+        unsigned smid;
+        asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+        const bool producer_here = *(volatile const int*)p.producer_sm == (int)smid + 1;
+        s_leave = producer_here && *(volatile const unsigned*)q.workers > 0u;
+        if (!s_leave)
+            atomicAdd(q.workers, 1u);
+    }
+    __syncthreads();
+    if (s_leave)
+        return;
+    __shared__ PairStage stage[8];
+    const int lane = threadIdx.x & 31;
+    unsigned long long its = 0, reb = 0;
+    for (;;) {
+        unsigned base = 0;
+        if (lane == 0)
+            base = atomicAdd(q.pull, 64u);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= q.n)
+            break;
+        // the lane's pixels: a runs, b waits; they swap places
+        PixRun<float> a, b;
+        unsigned apix = 0, bpix = 0;
+        auto dc = [&](unsigned pix, double& re, double& im) {
+            const int line = (int)(pix / (unsigned)p.W);
+            const int ix = (int)(pix - (unsigned)line * (unsigned)p.W);
+            re = (double)(2 * ix - p.W) * p.hs_m;
+            im = (double)(p.H - 2 * (p.row0 + line)) * p.hs_m;
+        };
+        auto load = [&](unsigned i, PixRun<float>& r, unsigned& pix) -> bool {
+            if (i >= q.n)
+                return false;
+            const unsigned e = q.in ? q.in[i] : (i | kEntryFresh);
+            pix = e & kEntryPixelMask;
+            double re, im;
+            dc(pix, re, im);
+            if (e & kEntryFresh)
+                pixel_start(r, re, im, p.hs_e, fold_ke<float>(p));
+            else
+                load_run(r, q.state + (size_t)pix * 2u, re, im, p.hs_e, fold_ke<float>(p));
+            return true;
+        };
+        bool arun = load(base + lane, a, apix), brun = load(base + 32u + lane, b, bpix);
+        uint32_t alast = a.wz + q.budget - 1u, blast = b.wz + q.budget - 1u;
+        const OrbitSnap snap = orbit_snapshot(p);
+        bool again_a = false, again_b = false;
+        while (__any_sync(0xffffffffu, arun || brun)) {
+            const bool same =
+                arun && brun && a.m == b.m && a.wz == b.wz && deep_state(a) && deep_state(b);
+            bool pair = same && (a.wz & 3u) == 1u;   // blocks start there
+            const bool align = same && !pair;
+            double ar = 0.0, ai = 0.0, br = 0.0, bi = 0.0;
+            if (pair) {
+                dc(apix, ar, ai);
+                dc(bpix, br, bi);
+            }
+            pair = deep_pairs(p, stage[threadIdx.x >> 5], pair, a, b,
+                              min(min(alast, blast), p.depth), snap.avail, (float)ar, (float)ai,
+                              (float)br, (float)bi);
+            // each alone: past what stopped the pair, or to the end
+#pragma unroll 1
+            for (int turn = 0; turn < 2; ++turn) {
+                if (arun && a.wz > alast) {
+                    arun = false;   // its budget is used up
+                    again_a = true;
+                    store_run(a, q.state + (size_t)apix * 2u);
+                } else if (arun) {
+                    const uint32_t to = pair    ? min(alast, a.wz + 15u)
+                                        : align ? min(alast, (a.wz + 3u) & ~3u)
+                                                : alast;
+                    double re, im;
+                    dc(apix, re, im);
+                    uint32_t count = 0;
+                    if (perturb_run<float, kOrbitSnapshot, MDZ_MANDELBROT>(
+                            p, a, re, im, p.hs_e, to, count, nullptr, snap) == 1) {
+                        arun = false;
+                        p.out[apix] = (int32_t)count;
+                        if (WANT_MAG)
+                            p.mag[apix] = a.mag;
+                        if (a.lost > p.lost_limit && p.flag_out)
+                            p.flag_out[atomicAdd(p.flag_out_count, 1u)] = apix;
+                        else
+                            its += count ? count : p.depth;
+                        reb += a.rebases;
+                    } else if (a.wz > alast || a.wz <= to) {
+                        // its budget is used up, or it waits for the orbit
+                        arun = false;
+                        again_a = true;
+                        store_run(a, q.state + (size_t)apix * 2u);
+                    }
+                }
+                const PixRun<float> r = a;
+                a = b;
+                b = r;
+                const unsigned x = apix;
+                apix = bpix;
+                bpix = x;
+                const uint32_t l = alast;
+                alast = blast;
+                blast = l;
+                const bool f = arun, g = again_a;
+                arun = brun;
+                brun = f;
+                again_a = again_b;
+                again_b = g;
+            }
+        }
+        queue_append(again_a, apix, q.out, q.out_count);
+        queue_append(again_b, bpix, q.out, q.out_count);
+    }
+    its = warp_sum_u64(its);
+    reb = warp_sum_u64(reb);
+    if (lane == 0) {
+        if (its)
+            atomicAdd(&p.sync->iter_sum, its);
+        if (reb)
+            atomicAdd(p.rebases, reb);
+    }
+}
+
 __global__ void frame_step_reset_kernel(unsigned* counters)
 {
     counters[0] = 0u;   // pull
@@ -2832,6 +3175,11 @@ int launch_orbit_stream(const OrbitLaunch& o, int* progress, cudaStream_t s, Don
     return MDZGPU_OK;
 }
 
+bool perturb_in_pairs(int num_sms, const PerturbLaunch& p, size_t n)
+{
+    return p.fractal == MDZ_MANDELBROT && p.att && p.hs_e < -160 && n >= (size_t)64 * 24 * num_sms;
+}
+
 int launch_perturb_step(int num_sms, const PerturbLaunch& p, const unsigned* in, unsigned n,
                         unsigned* out, unsigned* counters, uint4* state, unsigned budget,
                         cudaStream_t s, cudaEvent_t before, cudaEvent_t after)
@@ -2844,9 +3192,12 @@ int launch_perturb_step(int num_sms, const PerturbLaunch& p, const unsigned* in,
                              {(const void*)perturb_step_kernel<true, 0>,
                               (const void*)perturb_step_kernel<true, 1>,
                               (const void*)perturb_step_kernel<true, 2>}};
-    const void* fn = fns[mag ? 1 : 0][fr];
-    static int bps[2][3] = {{0, 0, 0}, {0, 0, 0}};
-    int& b = bps[mag ? 1 : 0][fr];
+    const bool pairs = perturb_in_pairs(num_sms, p, n);
+    const void* fn = pairs ? (mag ? (const void*)perturb_pairs_kernel<true>
+                                  : (const void*)perturb_pairs_kernel<false>)
+                           : fns[mag ? 1 : 0][fr];
+    static int bps[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    int& b = bps[mag ? 1 : 0][pairs ? 3 : fr];
     if (!b) {
         MDZ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, 256, 0));
         if (b < 1)
