@@ -15,12 +15,21 @@
 //    lanes.
 //  * Products (one general, two squares per iteration) are truncated like
 //    the one-thread kernel (partial products with i + j < NL - 2 skipped).
-//    The operands go to shared memory; lane l forms the 192-bit sums of the
-//    columns c = NL - 2 + l + G t (interleaved, so every lane gets short
-//    and long columns) with mad.lo.cc.u64 / madc.hi.cc.u64; the three
-//    64-bit parts of every column go back to shared memory shifted by 0, 1
-//    and 2 limbs and are added as distributed numbers (lane carries as
-//    above); the result is the window F .. F + 64 NL of that sum.
+//    The operands go to shared memory in blocks of four 32-bit words (two
+//    limbs).  A lane multiplies whole blocks: all pairs (p, q) with p + q = C,
+//    one tile, add up in seven 96-bit column sums in its registers, two 128-bit
+//    loads feeding 16 multiply-adds.  A square takes the pairs p < q doubled
+//    and the block p = q.  A tile's nine words go back to shared memory as
+//    three block-sized parts, shifted by 0, 1 and 2 blocks, and the parts of all
+//    tiles are added as three distributed numbers (lane carries as above); the
+//    result is the window F .. F + 64 NL of that sum.
+//
+// What bounds it is the integer multiplier, 1.1 SM cycles a warp for each
+// 32x32-bit product, and the lanes that wait for the group's longest tile
+// (tiles hold 1 to NL / 2 pairs; three rounds of G tiles at NL = 40 keep 75% of
+// the lanes at work).  64-bit products (mad.lo/hi.u64: a dozen instructions for
+// four 32-bit products, a load each) took 45.8 ms for a 96x64 view at 2176 bits,
+// this form 27.2 ms.
 //
 // The four (G = 8) or one (G = 32) pixels of a warp run in lock step: a
 // group whose pixel finishes writes its count and takes the next pixel
@@ -44,36 +53,45 @@ __device__ __forceinline__ unsigned long long warp_sum_its(unsigned long long v)
     return v;
 }
 
-__device__ __forceinline__ uint64_t mad_lo_cc(uint64_t a, uint64_t b, uint64_t c)
+// Column sums of a tile: 96 bits each (low 64, high 32), column k at word
+// weight k.
+struct TileSums {
+    uint64_t lo[7];
+    uint32_t hi[7];
+};
+
+// Adds the 16 products x_u y_v to the columns u + v.
+__device__ __forceinline__ void add_block(TileSums& s, const uint4& x, const uint4& y)
 {
-    uint64_t r;
-    asm volatile("mad.lo.cc.u64 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t madc_hi_cc(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t r;
-    asm volatile("madc.hi.cc.u64 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t addc_0(uint64_t a)
-{
-    uint64_t r;
-    asm volatile("addc.u64 %0, %1, 0;" : "=l"(r) : "l"(a));
-    return r;
+    const uint32_t a[4] = {x.x, x.y, x.z, x.w}, b[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            // (a 64-bit register pair: the two halves become one multiply-add)
+            asm("{.reg .u32 l, h;\n\t"
+                "mov.b64 {l, h}, %0;\n\t"
+                "mad.lo.cc.u32 l, %2, %3, l;\n\t"
+                "madc.hi.cc.u32 h, %2, %3, h;\n\t"
+                "addc.u32 %1, %1, 0;\n\t"
+                "mov.b64 %0, {l, h};}"
+                : "+l"(s.lo[u + v]), "+r"(s.hi[u + v]) : "r"(a[u]), "r"(b[v]));
+        }
 }
 
 template <int G, int Q>
 struct Mpw {
     static constexpr int NL = G * Q;          // limbs per number
-    static constexpr int QP = Q + 1;          // limbs per lane of the column sums
-    static constexpr int NP = G * QP;         // >= NL + 3 positions (G >= 4)
-    static_assert(G >= 4 && G <= 32 && (32 % G) == 0, "group of 4..32 lanes");
+    static constexpr int QP = Q + 1;          // limbs per lane of the tiles' sum
+    static constexpr int NP = G * QP;         // >= NL + 6 positions
+    static constexpr int NB = NL / 2;         // blocks of four words per number
+    static_assert(G >= 8 && G <= 32 && (32 % G) == 0, "group of 8..32 lanes");
+    static_assert(NL % 2 == 0 && NP % 2 == 0 && NP >= NL + 6, "whole blocks");
 
     // shared memory of one group
-    struct Smem {
+    struct alignas(16) Smem {
         uint64_t a[NL], b[NL];               // operands
-        uint64_t t0[NP], t1[NP], t2[NP];     // column-sum parts; position p = column NL-2+p
+        uint64_t t0[NP], t1[NP], t2[NP];     // tile parts; position p = limb NL-4+p
     };
 
     int pl;          // lane within the group
@@ -211,63 +229,88 @@ struct Mpw {
             if (!SQUARE)
                 sm->b[pl * Q + k] = b[k];
         }
-        // positions no column writes (see below) start at zero
-        if (pl == 0) {
-            sm->t1[0] = 0ull;
-            sm->t2[0] = 0ull;
-            sm->t2[1] = 0ull;
-        }
-#pragma unroll
-        for (int p = NL + 1 + pl; p < NP; p += G) {
-            sm->t0[p] = 0ull;
-            if (p >= NL + 2)
-                sm->t1[p] = 0ull;
-            if (p >= NL + 3)
-                sm->t2[p] = 0ull;
-        }
         __syncwarp();
-        const uint64_t* A = sm->a;
-        const uint64_t* B = SQUARE ? sm->a : sm->b;
-        constexpr int NC = NL + 1;                       // columns NL-2 .. 2NL-2
-        constexpr int T = (NC + G - 1) / G;
+        const uint4* A = (const uint4*)sm->a;
+        const uint4* B = SQUARE ? A : (const uint4*)sm->b;
+        uint4* T0 = (uint4*)sm->t0;
+        uint4* T1 = (uint4*)sm->t1;
+        uint4* T2 = (uint4*)sm->t2;
+        // tile t = 0 .. NB: blocks p + q = C = NB - 2 + t; of tile 0 only the
+        // upper limbs' products (i + j = NL - 2).  Every other round is dealt
+        // backwards, so that a lane's tiles even out.
+        constexpr int ROUNDS = (NB + 1 + G - 1) / G;
+#pragma unroll 1
+        for (int round = 0; round < ROUNDS; ++round) {
+            const int t = G * round + ((round & 1) ? G - 1 - pl : pl);
+            if (t > NB)
+                continue;
+            const int C = NB - 2 + t;
+            const uint32_t low = t ? 0xffffffffu : 0u;   // words 0 and 1 count
+            TileSums s;
 #pragma unroll
-        for (int t = 0; t < T; ++t) {
-            const int p = pl + G * t;
-            if (p < NC) {
-                const int c = NL - 2 + p;
-                const int ilo = c - (NL - 1) > 0 ? c - (NL - 1) : 0;
-                uint64_t s0 = 0ull, s1 = 0ull, s2 = 0ull;
-                if (SQUARE) {
-                    // off-diagonal terms i < j once, doubled, plus the diagonal
-                    const int ihi = (c - 1) >> 1;
-                    for (int i = ilo; i <= ihi; ++i) {
-                        const uint64_t x = A[i], y = A[c - i];
-                        s0 = mad_lo_cc(x, y, s0);
-                        s1 = madc_hi_cc(x, y, s1);
-                        s2 = addc_0(s2);
-                    }
-                    s2 = (s2 << 1) | (s1 >> 63);
-                    s1 = (s1 << 1) | (s0 >> 63);
-                    s0 <<= 1;
-                    if (!(c & 1)) {
-                        const uint64_t h = A[c >> 1];
-                        s0 = mad_lo_cc(h, h, s0);
-                        s1 = madc_hi_cc(h, h, s1);
-                        s2 = addc_0(s2);
-                    }
-                } else {
-                    const int ihi = c < NL - 1 ? c : NL - 1;
-                    for (int i = ilo; i <= ihi; ++i) {
-                        const uint64_t x = A[i], y = B[c - i];
-                        s0 = mad_lo_cc(x, y, s0);
-                        s1 = madc_hi_cc(x, y, s1);
-                        s2 = addc_0(s2);
-                    }
-                }
-                sm->t0[p] = s0;
-                sm->t1[p + 1] = s1;
-                sm->t2[p + 2] = s2;
+            for (int k = 0; k < 7; ++k)
+                s.lo[k] = s.hi[k] = 0u;
+            int p = C - (NB - 1) > 0 ? C - (NB - 1) : 0;
+            const int last = SQUARE ? (C - 1) >> 1 : C - p;
+#pragma unroll 1
+            for (; p <= last; ++p) {
+                uint4 x = A[p], y = B[C - p];
+                x.x &= low;
+                x.y &= low;
+                y.x &= low;
+                y.y &= low;
+                add_block(s, x, y);
             }
+            if (SQUARE) {
+                // the pairs' sums doubled, then the block p = q
+#pragma unroll
+                for (int k = 0; k < 7; ++k) {
+                    s.hi[k] = __funnelshift_l((uint32_t)(s.lo[k] >> 32), s.hi[k], 1);
+                    s.lo[k] <<= 1;
+                }
+                if (!(C & 1)) {
+                    uint4 x = A[C >> 1];
+                    x.x &= low;
+                    x.y &= low;
+                    add_block(s, x, x);
+                }
+            }
+            // the tile as nine words: the columns' low, middle and high words
+            // are numbers shifted by one word each
+            auto w0 = [&](int k) { return (uint32_t)s.lo[k]; };
+            auto w1 = [&](int k) { return (uint32_t)(s.lo[k] >> 32); };
+            uint32_t r[9];
+            r[0] = w0(0);
+            asm volatile("add.cc.u32 %0, %1, %2;" : "=r"(r[1]) : "r"(w0(1)), "r"(w1(0)));
+#pragma unroll
+            for (int k = 2; k < 7; ++k)
+                asm volatile("addc.cc.u32 %0, %1, %2;"
+                             : "=r"(r[k]) : "r"(w0(k)), "r"(w1(k - 1)));
+            asm volatile("addc.cc.u32 %0, %1, 0;" : "=r"(r[7]) : "r"(w1(6)));
+            asm volatile("addc.u32 %0, 0, 0;" : "=r"(r[8]));
+            asm volatile("add.cc.u32 %0, %0, %1;" : "+r"(r[2]) : "r"(s.hi[0]));
+#pragma unroll
+            for (int k = 3; k < 8; ++k)
+                asm volatile("addc.cc.u32 %0, %0, %1;" : "+r"(r[k]) : "r"(s.hi[k - 2]));
+            asm volatile("addc.u32 %0, %0, %1;" : "+r"(r[8]) : "r"(s.hi[6]));
+            T0[t] = make_uint4(r[0], r[1], r[2], r[3]);
+            T1[t + 1] = make_uint4(r[4], r[5], r[6], r[7]);
+            T2[t + 2] = make_uint4(r[8], 0u, 0u, 0u);
+        }
+        // blocks no tile writes
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        if (pl == 0) {
+            T1[0] = zero;
+            T2[0] = zero;
+            T2[1] = zero;
+        }
+#pragma unroll
+        for (int q = NB + 1 + pl; q < NP / 2; q += G) {
+            T0[q] = zero;
+            if (q >= NB + 2)
+                T1[q] = zero;
+            if (q >= NB + 3)
+                T2[q] = zero;
         }
         __syncwarp();
         uint64_t u0[QP], u1[QP], u2[QP];
@@ -284,13 +327,13 @@ struct Mpw {
         for (int k = 0; k < QP; ++k)
             sm->t0[pl * QP + k] = u0[k];
         __syncwarp();
-        // r[k] = bits F - SQ + 64 k .. of the sum: position k + 1 holds bit F
-        // at offset 56 (F = 64 NL - 8, position 1 = column NL - 1)
+        // r[k] = bits F - SQ + 64 k .. of the sum: position k + 3 holds bit F
+        // at offset 56 (F = 64 NL - 8, position 3 = limb NL - 1)
         constexpr int SH = 56 - SQ;
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
             const int g = pl * Q + k;
-            const uint64_t lo = sm->t0[g + 1], hi = sm->t0[g + 2];
+            const uint64_t lo = sm->t0[g + 3], hi = sm->t0[g + 4];
             r[k] = (lo >> SH) | (hi << (64 - SH));
         }
         __syncwarp();
