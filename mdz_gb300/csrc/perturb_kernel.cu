@@ -1772,6 +1772,10 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
     const uint32_t last = wz_last < p.depth ? wz_last : p.depth;
     uint32_t wz = r.wz;
     bool blocked = false;
+    // the FP32 Mandelbrot pass stops a pixel once it has lost more bits than
+    // the pass allows: the FP64 pass redoes it from the start, whatever its
+    // remaining iterations would give
+    auto handed_on = [&]() { return !kTrack && r.lost > p.lost_limit && p.flag_out != nullptr; };
     while (wz <= last) {
         bool attention = false;
         T dd;   // |t|^2 after the step
@@ -1993,6 +1997,12 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
                     rebase_fp64<T>(p, m, st, dcf_r, dcf_i, dce, rebase_lost, false);
                     if (kTrack)
                         fold_rebase_err<T>(p, m, st, e0);
+                    if (handed_on()) {
+                        r.mag = 0.f;
+                        count = 0;
+                        ++r.rebases;
+                        return 1;
+                    }
                     m = rebase_to(wz);
                     if (kTwo)
                         K = avail = m ? q0 + *p.q_len : *p.orbit_len;
@@ -2123,6 +2133,12 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
             if (rebase_fp64<T>(p, m, st, dcf_r, dcf_i, dce, rebase_lost, true)) {
                 if (kTrack)
                     fold_rebase_err<T>(p, m, st, e0);
+                if (handed_on()) {
+                    r.mag = 0.f;
+                    count = 0;
+                    ++r.rebases;
+                    return 1;
+                }
                 m = rebase_to(wz + 1);
                 if (kTwo)
                     K = avail = m ? q0 + *p.q_len : *p.orbit_len;
