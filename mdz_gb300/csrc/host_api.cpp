@@ -1013,6 +1013,7 @@ static int perturb_common(mdzgpu_ctx* ctx, const mdzgpu_frame* f, const mdzgpu_m
                 cudaEventDestroy(evo);
                 return rc;
             }
+            launches += mp_list_launches(w) - 1;
             h2d_extra = (int64_t)tab.size() * 4;
         }
     }

@@ -148,6 +148,8 @@ struct MpLaunch {
     const unsigned* list = nullptr;
     const unsigned* list_count = nullptr;
     float* mag = nullptr;   // |z|^2 at escape (FP32), when non-null
+    // lists of at most this many pixels run one pixel a block (set by the launch)
+    unsigned pixel_limit = 0;
     DoneSignal done;        // optional: stores 1 when the launch is complete
                             // (3 when it also reached the list's end)
     // list pass in chunks: this launch takes tiles tile_base + [0, tile_limit)
@@ -155,7 +157,20 @@ struct MpLaunch {
     // polls a bounded wait of the fused launch makes before it gives up
     int spin_limit = kSpinLimit;
 };
+// Lists of at most this many pixels an SM go to mp_pixel_kernel: a block's
+// iteration takes 0.8 us at N = 8, 0.9 at 16, 1.25 at 34, and each further
+// pixel an SM adds 0.06 to 0.1; a thread's takes 0.47, 1.23, 4.2.  (16000
+// iterations at N = 34, 2.8 pixels an SM: 20.1 ms and 68.2, 8.5: 25.9 and 68.5;
+// 10000 at N = 16, 1.4: 9.1 and 12.5, 5.3: 11.9 and 12.6; at N = 8, 2.6: 12.3
+// and 7.3 for 15000.)
+template <int N>
+constexpr int pixel_list_per_sm()
+{
+    return N >= 34 ? 32 : N >= 28 ? 18 : N >= 24 ? 10 : N >= 20 ? 7 : N >= 16 ? 5 : 0;
+}
 int launch_mp(mdzgpu_ctx* ctx, const MpLaunch& p, cudaStream_t s);
+// Kernels launch_mp launches for a list's first chunk.
+int mp_list_launches(int words);
 bool mp_words_supported(int words);
 // Word counts the multi-limb kernel is compiled for (one translation unit
 // each; the build reads this list).

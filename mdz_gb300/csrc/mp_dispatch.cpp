@@ -38,6 +38,16 @@ int launch_mp(mdzgpu_ctx* ctx, const MpLaunch& p, cudaStream_t s)
     }
 }
 
+int mp_list_launches(int words)
+{
+#define MDZ_CASE(n) \
+    if (words == n) \
+        return pixel_list_per_sm<n>() > 0 ? 2 : 1;
+    MDZ_MP_WORDS_LIST(MDZ_CASE)
+#undef MDZ_CASE
+    return 1;
+}
+
 int preload_mp_kernels()
 {
     int rc = MDZGPU_OK;

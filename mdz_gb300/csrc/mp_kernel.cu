@@ -167,7 +167,10 @@ __global__ void __launch_bounds__(kFrameBlock, frame_blocks_per_sm<N>())
     const int tiles_x = (p.W + kTileW - 1) / kTileW;
     const int tiles_y = (p.nrows + kTileH - 1) / kTileH;
     const unsigned list_n = p.list ? *p.list_count : 0u;
-    const unsigned total = p.list ? (list_n + 31u) / 32u : (unsigned)tiles_x * (unsigned)tiles_y;
+    const unsigned listed = (list_n + 31u) / 32u;
+    // (a short list is mp_pixel_kernel's)
+    const unsigned total = p.list ? (list_n <= p.pixel_limit ? 0u : listed)
+                                  : (unsigned)tiles_x * (unsigned)tiles_y;
     unsigned long long its = 0;
     TileFeed feed;
     bool active = false;   // this lane iterates a pixel
@@ -254,7 +257,249 @@ __global__ void __launch_bounds__(kFrameBlock, frame_blocks_per_sm<N>())
     if (lane == 0 && its)
         atomicAdd(&p.sync->iter_sum, its);
     if (p.done.count)
-        done_signal(p.done, (unsigned long long)p.tile_base + p.tile_limit >= total ? 3 : 1);
+        done_signal(p.done, (unsigned long long)p.tile_base + p.tile_limit >= listed ? 3 : 1);
+}
+
+// ---- short lists: one pixel a block ----
+//
+// The perturbation hands a few hundred to a few thousand pixels to the
+// multi-limb pass, to run thousands of iterations each; one thread a pixel
+// takes 1.2 us an iteration at N = 16 and 4.2 us at N = 34 however few they
+// are.  Here a block of 4 (N + 1) threads iterates one pixel, with the same
+// truncated products, so the same counts:
+//
+//  1. Thread 4 k + s forms one column sum, column N-2+k, in 96 bits: s = 0, 1
+//     half of the general product's terms each, s = 2, 3 those of the squares
+//     of wim, wre (i < j once, doubled, and the diagonal).
+//  2. Two warps, a 64-bit limb a lane, add up the columns: warp 0 the product,
+//     and from it the next wim; warp 1 the squares, and from them the escape
+//     test and the next wre.  Carries between lanes come from two ballots
+//     (generate / propagate, as in mpw_kernel.cu).
+//
+// What bounds it is latency (two barriers and two warps' chains an iteration)
+// for a pixel an SM, issue for more.
+template <int N>
+__host__ __device__ constexpr int pixel_threads()
+{
+    return 4 * (N + 1) <= 64 ? 64 : (4 * (N + 1) + 31) / 32 * 32;
+}
+
+// x + y + c0 over the warp's limbs, lane 0 lowest.
+__device__ __forceinline__ uint64_t warp_add(uint64_t x, uint64_t y, unsigned c0)
+{
+    const uint64_t s = x + y;
+    const unsigned g = __ballot_sync(0xffffffffu, s < x);
+    const unsigned p = __ballot_sync(0xffffffffu, s == ~0ull);
+    const uint64_t c = ((uint64_t)g + (g | p) + c0) ^ p;
+    return s + ((c >> (threadIdx.x & 31)) & 1u);
+}
+
+// c + x or, where neg, c - x.
+__device__ __forceinline__ uint64_t warp_add_signed(uint64_t c, uint64_t x, bool neg)
+{
+    return warp_add(c, neg ? ~x : x, neg);
+}
+
+template <int N>
+__global__ void __launch_bounds__(pixel_threads<N>()) mp_pixel_kernel(MpLaunch p)
+{
+    constexpr int NL = N / 2;
+    constexpr int NC = N + 1;              // columns N-2 .. 2N-2
+    __shared__ uint64_t z64[2][NL];        // |wim|, |wre|
+    __shared__ uint4 col[3][NC + 3];       // column k at [k + 2]: wre wim, wim^2, wre^2
+    __shared__ uint32_t sign[2];           // sign masks of wim, wre
+    __shared__ uint64_t top[2];            // signed top limbs of the next wim, wre
+    __shared__ int state;                  // 1: done
+    __shared__ uint32_t count, next;
+    __shared__ float mag;
+    const unsigned list_n = *p.list_count;
+    if (list_n > p.pixel_limit)
+        return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool ship = p.fractal == MDZ_BURNING_SHIP;
+    const bool celtic = p.fractal == MDZ_GENERALIZED_CELTIC;
+    const bool variant = p.fractal == MDZ_VARIANT;
+    // this thread's column sum: terms i0 .. i0 + len - 1
+    const int k = tid >> 2, set = tid & 3;
+    const int c = N - 2 + k;
+    const int ilo = c - (N - 1) > 0 ? c - (N - 1) : 0;
+    const int all = (c < N - 1 ? c : N - 1) - ilo + 1;   // terms of the product
+    const int i0 = set == 1 ? ilo + (all + 1) / 2 : ilo;
+    const int len = k >= NC ? 0 : set == 0 ? (all + 1) / 2 : set == 1 ? all / 2
+                                                           : ((c - 1) >> 1) - ilo + 1;
+    const int steps = __reduce_max_sync(0xffffffffu, len);
+    const uint32_t* zim = (const uint32_t*)z64[0];
+    const uint32_t* zre = (const uint32_t*)z64[1];
+    const uint32_t* pa = (set == 2 ? zim : zre) + i0;
+    const uint32_t* pb = (set == 3 ? zre : zim) + (c - i0);
+    // columns that do not exist
+    for (int j = tid; j < 9; j += blockDim.x)
+        col[j / 3][j % 3 < 2 ? j % 3 : NC + 2] = make_uint4(0u, 0u, 0u, 0u);
+
+    // the sum of a product's columns from word N-2 on, 64 bits a lane
+    auto limbs = [&](const uint4* cs) -> uint64_t {
+        const bool in = lane <= NL;
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        const uint4 A = in ? cs[2 * lane + 2] : zero, B = in ? cs[2 * lane + 3] : zero;
+        const uint4 C = in ? cs[2 * lane] : zero, D = in ? cs[2 * lane + 1] : zero;
+        const uint64_t x = (uint64_t)A.y << 32 | A.x, y = (uint64_t)B.x << 32;
+        const uint64_t z = (uint64_t)C.z + D.y, w = (uint64_t)D.z << 32;
+        uint64_t s = x + y;
+        unsigned v = s < x;
+        s += z;
+        v += s < z;
+        s += w;
+        v += s < w;
+        unsigned from = __shfl_up_sync(0xffffffffu, v, 1);
+        if (lane == 0)
+            from = 0;
+        return warp_add(s, from, 0);
+    };
+    // that sum's bits from 32 + SH on: floor(P / 2^F) for SH = 24, of 2 P for 23
+    auto extract = [&](uint64_t s, int sh) -> uint64_t {
+        const uint64_t up = __shfl_down_sync(0xffffffffu, s, 1);
+        return lane < NL ? s >> (32 + sh) | up << (32 - sh) : 0ull;
+    };
+    auto big = [](uint64_t t) {
+        const int32_t h = (int32_t)(t >> 32);
+        return h >= 0x08000000 || h < -0x08000000;
+    };
+    auto top_float = [](uint64_t t) {
+        return (float)(int32_t)(t >> 32) * 5.9604645e-8f /* 2^-24 */
+               + (float)(uint32_t)t * 1.3877788e-17f /* 2^-56 */;
+    };
+    // |v| to shared memory, its sign mask and signed top limb beside it
+    auto publish = [&](uint64_t v, int part) {
+        const uint64_t t = __shfl_sync(0xffffffffu, v, NL - 1);
+        const bool neg = (int64_t)t < 0;
+        if (neg)
+            v = warp_add(~v, 0ull, 1);
+        if (lane < NL)
+            z64[part][lane] = v;
+        if (lane == 0) {
+            sign[part] = neg ? 0xffffffffu : 0u;
+            top[part] = t;
+        }
+    };
+    unsigned long long its = 0;
+    for (;;) {
+        if (tid == 0) {
+            const unsigned t = atomicAdd(&p.sync->tile_counter, 1u);
+            next = t < list_n ? p.list[t] : 0xffffffffu;
+            state = 0;
+        }
+        __syncthreads();
+        const unsigned pix = next;
+        if (pix == 0xffffffffu)
+            break;
+        // warp 0: y and c_im, warp 1: x and c_re
+        uint64_t cst = 0;
+        if (warp < 2) {
+            const unsigned row = pix / (unsigned)p.W, ix = pix - row * (unsigned)p.W;
+            const uint64_t* v = (const uint64_t*)(warp ? p.xs + (size_t)ix * N
+                                                       : p.ys + (size_t)row * N);
+            const uint64_t z = lane < NL ? v[lane] : 0ull;
+            cst = z;
+            if (p.family == MDZ_FAMILY_JULIA)
+                cst = lane < NL ? ((const uint64_t*)(p.julia + (warp ? 0 : N)))[lane] : 0ull;
+            publish(z, warp);
+        }
+        uint32_t wz = 0;   // iterations done
+        for (;;) {
+            __syncthreads();
+            if (wz && state == 0 && (big(top[0]) || big(top[1]))) {
+                if (tid == 0) {
+                    const float a = top_float(top[1]), b = top_float(top[0]);
+                    mag = a * a + b * b;
+                    count = wz;
+                }
+                break;
+            }
+            if (state)
+                break;
+            // column sums
+            {
+                uint32_t w0 = 0, w1 = 0, w2 = 0;
+#pragma unroll 4
+                for (int j = 0; j < steps; ++j) {
+                    const uint32_t x = j < len ? pa[j] : 0u, y = j < len ? pb[-j] : 0u;
+                    asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
+                        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+                        "addc.u32 %2, %2, 0;"
+                        : "+r"(w0), "+r"(w1), "+r"(w2) : "r"(x), "r"(y));
+                }
+                if (set >= 2) {
+                    w2 = __funnelshift_l(w1, w2, 1);
+                    w1 = __funnelshift_l(w0, w1, 1);
+                    w0 <<= 1;
+                    const uint32_t h = (k < NC && !(c & 1)) ? (set == 2 ? zim : zre)[c >> 1] : 0u;
+                    asm("mad.lo.cc.u32 %0, %3, %3, %0;\n\t"
+                        "madc.hi.cc.u32 %1, %3, %3, %1;\n\t"
+                        "addc.u32 %2, %2, 0;"
+                        : "+r"(w0), "+r"(w1), "+r"(w2) : "r"(h));
+                }
+                // the product's halves are neighbours
+                const uint32_t v0 = __shfl_xor_sync(0xffffffffu, w0, 1);
+                const uint32_t v1 = __shfl_xor_sync(0xffffffffu, w1, 1);
+                const uint32_t v2 = __shfl_xor_sync(0xffffffffu, w2, 1);
+                if (set == 0)
+                    asm("add.cc.u32 %0, %0, %3;\n\t"
+                        "addc.cc.u32 %1, %1, %4;\n\t"
+                        "addc.u32 %2, %2, %5;"
+                        : "+r"(w0), "+r"(w1), "+r"(w2) : "r"(v0), "r"(v1), "r"(v2));
+                if (k < NC && set != 1)
+                    col[set ? set - 1 : 0][k + 2] = make_uint4(w0, w1, w2, 0u);
+            }
+            const uint32_t sre = sign[1], sim = sign[0];
+            __syncthreads();
+            ++wz;
+            if (warp == 0) {
+                // wim = 2.0 * wre * wim + c_im   (burning ship: 2 |wre wim| + c_im)
+                const uint64_t t = extract(limbs(col[0]), 23);
+                publish(warp_add_signed(cst, t, !ship && sre != sim), 0);
+            } else if (warp == 1) {
+                const uint64_t wim2 = extract(limbs(col[1]), 24);
+                const uint64_t wre2 = extract(limbs(col[2]), 24);
+                // |z|^2 > 4 (not of z_0 = c)
+                const uint64_t ta = __shfl_sync(0xffffffffu, wim2, NL - 1);
+                const uint64_t tb = __shfl_sync(0xffffffffu, wre2, NL - 1);
+                const uint32_t sum = (uint32_t)(ta >> 32) + (uint32_t)(tb >> 32);
+                bool over = sum > 0x04000000u;
+                if (sum - 0x03ffffffu <= 1u) {
+                    const uint64_t s = warp_add(wim2, wre2, 0);
+                    const uint64_t t = __shfl_sync(0xffffffffu, s, NL - 1);
+                    const bool low = __any_sync(0xffffffffu, lane < NL - 1 ? s != 0ull
+                                                                           : lane == NL - 1
+                                                                                 && (uint32_t)s);
+                    over = (uint32_t)(t >> 32) > 0x04000000u
+                           || ((uint32_t)(t >> 32) == 0x04000000u && low);
+                }
+                over = over && wz > 1;
+                if (over || wz > p.depth) {
+                    if (lane == 0) {
+                        state = 1;
+                        count = over ? wz - 1 : 0u;
+                        mag = top_float(ta) + top_float(tb);
+                    }
+                } else {
+                    // wre = wre2 - wim2 + c_re       (celtic: |wre2 - wim2| + c_re)
+                    const uint64_t d = warp_add(wre2, ~wim2, 1);
+                    const bool neg = (int64_t)__shfl_sync(0xffffffffu, d, NL - 1) < 0;
+                    const bool fold = neg && (celtic || (variant && (wz & 1u)));
+                    publish(warp_add_signed(cst, d, fold), 1);
+                }
+            }
+        }
+        if (tid == 0) {
+            p.out[pix] = (int32_t)count;
+            if (p.mag)
+                p.mag[pix] = mag;
+            its += count ? count : p.depth;
+        }
+        __syncthreads();
+    }
+    if (tid == 0 && its)
+        atomicAdd(&p.sync->iter_sum, its);
 }
 
 // Serving: one step of the multi-limb method over its mixed work queue
@@ -403,6 +648,20 @@ int typed_blocks_per_sm(int* out)
     return MDZGPU_OK;
 }
 
+template <int N>
+int pixel_blocks_per_sm(int* out)
+{
+    static int blocks_per_sm = 0;
+    if (!blocks_per_sm) {
+        int b = 0;
+        MDZ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, mp_pixel_kernel<N>,
+                                                                   pixel_threads<N>(), 0));
+        blocks_per_sm = b < 1 ? 1 : b;
+    }
+    *out = blocks_per_sm;
+    return MDZGPU_OK;
+}
+
 template <int N, int FRACTAL, bool JULIA>
 int launch_typed(mdzgpu_ctx* ctx, const MpLaunch& p, cudaStream_t s)
 {
@@ -428,8 +687,23 @@ int launch_typed(mdzgpu_ctx* ctx, const MpLaunch& p, cudaStream_t s)
 }  // namespace
 
 template <int N>
-int launch_words(mdzgpu_ctx* ctx, const MpLaunch& p, cudaStream_t s)
+int launch_words(mdzgpu_ctx* ctx, const MpLaunch& frame, cudaStream_t s)
 {
+    MpLaunch p = frame;
+    p.pixel_limit = 0;
+    if (pixel_list_per_sm<N>() > 0 && p.list && p.tile_base == 0) {
+        // both kernels look at the list's length, which only the device knows,
+        // and one of them leaves; a short list is done in the first chunk (a
+        // later chunk means it was longer than the first one)
+        p.pixel_limit = (unsigned)(pixel_list_per_sm<N>() * ctx->num_sms);
+        constexpr int threads = pixel_threads<N>();
+        int b = 0;
+        if (int rc = pixel_blocks_per_sm<N>(&b))
+            return rc;
+        const long pixels = std::min((long)p.W * p.nrows, (long)p.pixel_limit);
+        mp_pixel_kernel<N><<<(unsigned)std::min(pixels, (long)ctx->num_sms * b), threads, 0, s>>>(p);
+        MDZ_CUDA_TRY(cudaGetLastError());
+    }
     const bool julia = p.family == MDZ_FAMILY_JULIA;
     switch (p.fractal) {
     case MDZ_BURNING_SHIP:
@@ -472,7 +746,7 @@ int launch_serve_mp_words(ServeDev* d, int mp_class, int num_sms, cudaStream_t s
 template <int N>
 int preload_words()
 {
-    int b = 0, rc = MDZGPU_OK;
+    int b = 0, rc = pixel_blocks_per_sm<N>(&b);
     for (int j = 0; j < 2 && !rc; ++j) {
         const bool julia = j == 1;
         rc = julia ? typed_blocks_per_sm<N, MDZ_MANDELBROT, true>(&b)

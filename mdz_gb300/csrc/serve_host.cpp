@@ -1046,10 +1046,11 @@ int Server::launch_escalation(const std::shared_ptr<Req>& r, bool mp_pass)
         q.tile_limit = chunk;
         rc = launch_mp(&shape, q, es);
     }
+    const int launched = mp_pass && r->esc_base == 0 ? mp_list_launches(r->words) : 1;
     r->esc_base += chunk;
     if (!rc) {
         std::lock_guard<std::mutex> lk(mu);
-        st.launches += 1;
+        st.launches += launched;
     }
     return rc;
 }
