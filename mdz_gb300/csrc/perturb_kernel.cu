@@ -2308,25 +2308,53 @@ __device__ __forceinline__ void pixel_tiles(const PerturbLaunch& p)
 // kListRefill lanes are idle (counts differ by thousands of iterations from
 // pixel to pixel); chunks of a multiple of four iterations keep the lanes'
 // every-fourth-iteration checks together.  Bound by the FP64 pipe: twelve
-// DFMAs an iteration, 70-77% busy (640x480 at 2^-100 to depth 15000, 1.0e9
-// iterations: 93-118 ms with 30 FP64 instructions an iteration and whole tiles,
-// 42.4 ms now; with 4 blocks of 4 warps an SM, 46.3 with 3, 44.7 with 2, 56
-// with 1).
+// DFMAs an iteration (640x480 at 2^-100 to depth 15000, 127 000 pixels and
+// 1.0e9 iterations: 93-118 ms with 30 FP64 instructions an iteration and whole
+// tiles, 28.5 now), until an SM has less than about eight warps of pixels left;
+// then by an iteration's latency, 0.8 us.
+//
+// So Mandelbrot's pass runs as many pixels at once as the registers allow, one
+// block an SM, whose warps merge as pixels finish: no pixel starts late, and
+// the pipe stays full until few are left.  (The same list: 42.4 ms in blocks of
+// 4 warps, 4 an SM, without merging, when the last 40% of the time ran 7 lanes
+// a warp; one block of 16 warps 38, of 24 32, of 28 28.5, of 32 28.7; 24 warps
+// without merging 53.)  The folded formulas' pixels are mostly direct ones:
+// 4 blocks of 4 warps (480x270 burning ship at 2^-300: 11.3 ms; a block of 24
+// 13).
+constexpr int kListMove = 128;   // pixels moved to other warps at a time
 constexpr int kListChunk = 64;
 constexpr int kListRefill = 6;
-constexpr int kListBlock = 128;
-constexpr int kListBlocksPerSm = 4;
+template <int FR>
+__host__ __device__ constexpr int list_block()
+{
+    return FR == MDZ_MANDELBROT ? 896 : 128;
+}
+template <int FR>
+__host__ __device__ constexpr int list_blocks_per_sm()
+{
+    return FR == MDZ_MANDELBROT ? 1 : 4;
+}
 
 template <bool WANT_MAG, int FR, bool JU>
 __device__ __forceinline__ void list_pixels(const PerturbLaunch& p)
 {
-    __shared__ unsigned listed[kListBlock / 32][32];   // the warp's current 32 entries
+    constexpr int kWarps = list_block<FR>() / 32;
+    __shared__ unsigned listed[kWarps][32];   // the warp's current 32 entries
     // folded formulas: pixels to iterate directly.  They wait here until there
     // are 32, while their lanes go on with the list: run at once, each lane's
     // thousands of direct iterations would hold up the other 31.
     constexpr bool kDirect = FR != MDZ_MANDELBROT;
-    __shared__ DirectPixel direct[kDirect ? kListBlock / 32 : 1][kDirect ? 64 : 1];
+    __shared__ DirectPixel direct[kDirect ? kWarps : 1][kDirect ? 64 : 1];
     int nd = 0;
+    // (not the folded formulas: their warps end with direct pixels, which
+    // are not to wait for one another)
+    constexpr bool kMerge = !kDirect;
+    __shared__ LaneMerge<kWarps> merge;
+    __shared__ uint32_t moved[kMerge ? 15 : 1][kMerge ? kListMove : 1];
+    int kept = kWarps;
+    bool dry = false;   // the list is used up
+    if (kMerge)
+        merge.init();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned list_n = *p.list_in_count;
     const unsigned total = (list_n + 31u) / 32u;
@@ -2336,7 +2364,63 @@ __device__ __forceinline__ void list_pixels(const PerturbLaunch& p)
     unsigned pix = 0;
     PixRun<double> r;
     double dcm_r = 0.0, dcm_i = 0.0;
+    // dc = ((2 ix - W) hs, (H - 2 line) hs), hs = half pixel spacing
+    auto set_dc = [&]() {
+        const int lrow = (int)(pix / (unsigned)p.W);
+        const int ix = (int)(pix - (unsigned)lrow * (unsigned)p.W);
+        dcm_r = (double)(2 * ix - p.W) * p.hs_m;
+        dcm_i = (double)(p.H - 2 * (p.row0 + lrow)) * p.hs_m;
+    };
     for (;;) {
+        if constexpr (kMerge) {
+            if (dry && merge.look(feed, active, kept)
+                && !merge.merge(
+                    feed, active, kept, kListMove,
+                    [&](int k) {
+                        int j = 0;
+                        auto put = [&](uint32_t w) { moved[j++][k] = w; };
+                        auto put64 = [&](double v) {
+                            put((uint32_t)__double2loint(v));
+                            put((uint32_t)__double2hiint(v));
+                        };
+                        put64(r.st.tr);
+                        put64(r.st.ti);
+                        put64(r.st.e2);
+                        put((uint32_t)r.st.e);
+                        put((uint32_t)r.m);
+                        put(r.wz);
+                        put(__float_as_uint(r.lost));
+                        put(r.rebases);
+                        put(__float_as_uint(r.mag));
+                        put(pix);
+                    },
+                    [&](int k) {
+                        int j = 0;
+                        auto get = [&]() { return moved[j++][k]; };
+                        auto get64 = [&]() {
+                            const uint32_t lo = get(), hi = get();
+                            return __hiloint2double((int)hi, (int)lo);
+                        };
+                        r.st.tr = get64();
+                        r.st.ti = get64();
+                        r.st.e2 = get64();
+                        r.st.e = (int)get();
+                        r.m = (int)get();
+                        r.wz = get();
+                        r.lost = __uint_as_float(get());
+                        r.rebases = get();
+                        r.mag = __uint_as_float(get());
+                        pix = get();
+                        r.st.ke = fold_ke<double>(p);
+                        r.st.tt = sqr_bits(r.st.ti);
+                        if (JU)
+                            dcm_r = dcm_i = 0.0;
+                        else
+                            set_dc();
+                        refresh_scale(r.st, dcm_r, dcm_i, p.hs_e);
+                    }))
+                break;
+        }
         bool fresh = false;
         feed_lanes(
             feed, !active,
@@ -2354,11 +2438,7 @@ __device__ __forceinline__ void list_pixels(const PerturbLaunch& p)
                 fresh = true;
             });
         if (fresh) {
-            const int lrow = (int)(pix / (unsigned)p.W);
-            const int ix = (int)(pix - (unsigned)lrow * (unsigned)p.W);
-            // dc = ((2 ix - W) hs, (H - 2 line) hs), hs = half pixel spacing
-            dcm_r = (double)(2 * ix - p.W) * p.hs_m;
-            dcm_i = (double)(p.H - 2 * (p.row0 + lrow)) * p.hs_m;
+            set_dc();
             pixel_start(r, dcm_r, dcm_i, p.hs_e, fold_ke<double>(p));
             if (JU) {
                 // Julia: the offset is the first delta, at V_0; no dc in the steps
@@ -2385,6 +2465,15 @@ __device__ __forceinline__ void list_pixels(const PerturbLaunch& p)
                 nd = from;
                 __syncwarp();
             }
+        }
+        if constexpr (kMerge) {
+            if (!feed.left && !feed.more && !dry) {
+                dry = true;
+                if (lane == 0)
+                    merge.set_dry();
+            }
+            if (!any)
+                continue;
         }
         if (!any)
             break;
@@ -2424,6 +2513,11 @@ __device__ __forceinline__ void list_pixels(const PerturbLaunch& p)
                 if (nd >= 32)
                     break;
             }
+            if (kMerge && (dry || merge.is_dry())) {
+                dry = true;
+                feed.more = false;
+                break;
+            }
         } while (__popc(__ballot_sync(0xffffffffu, !active)) < enough);
     }
     its = warp_sum_u64(its);
@@ -2436,7 +2530,7 @@ __device__ __forceinline__ void list_pixels(const PerturbLaunch& p)
 }
 
 template <class T, bool WANT_MAG, bool LIST, int FR, bool JU>
-__global__ void __launch_bounds__(LIST ? kListBlock : 256) perturb_kernel(PerturbLaunch p)
+__global__ void __launch_bounds__(LIST ? list_block<FR>() : 256) perturb_kernel(PerturbLaunch p)
 {
     if constexpr (LIST)
         list_pixels<WANT_MAG, FR, JU>(p);
@@ -3273,7 +3367,7 @@ int pass_blocks_per_sm(int* out)
     if (!bps) {
         int b = 0;
         MDZ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &b, perturb_kernel<T, WANT_MAG, LIST, FR, JU>, LIST ? kListBlock : 256, 0));
+            &b, perturb_kernel<T, WANT_MAG, LIST, FR, JU>, LIST ? list_block<FR>() : 256, 0));
         bps = b < 1 ? 1 : b;
     }
     *out = bps;
@@ -3286,11 +3380,12 @@ int launch_pass_fr(mdzgpu_ctx* ctx, const PerturbLaunch& p, cudaStream_t s, long
     int bps = 1;
     if (int rc = pass_blocks_per_sm<T, WANT_MAG, LIST, FR, JU>(&bps))
         return rc;
-    if (LIST && bps > kListBlocksPerSm)
-        bps = kListBlocksPerSm;
+    if (LIST && bps > list_blocks_per_sm<FR>())
+        bps = list_blocks_per_sm<FR>();
     long grid = (long)ctx->num_sms * bps;
-    const int threads = LIST ? kListBlock : 256;
-    const long blocks_needed = (work_items + threads / 32 - 1) / (threads / 32);
+    const int threads = LIST ? list_block<FR>() : 256;
+    const long blocks_needed = std::max((work_items + threads / 32 - 1) / (threads / 32),
+                                        LIST ? std::min(work_items, (long)ctx->num_sms) : 1L);
     if (grid > blocks_needed)
         grid = blocks_needed;
     if (grid < 1)
