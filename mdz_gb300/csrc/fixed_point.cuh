@@ -60,7 +60,8 @@ struct Columns {
 // Row I: a_j b for j = J0 .. N-1, into columns I + J0 .. I + N.  A chain
 // that ends with j = N-1 carries nothing out (the sum of rows 0..I is below
 // 2^(32 (I + 1 + N))); one that ends with j = N-2 carries into column I + N,
-// where its accumulator is still zero.
+// where its accumulator is still zero.  (Both hold for any subset of the rows,
+// taken in order.)
 template <int N, int I, int J0>
 __device__ __forceinline__ void row(Columns<N>& s, const uint32_t (&a)[N], uint32_t b)
 {
@@ -78,13 +79,14 @@ __device__ __forceinline__ void row(Columns<N>& s, const uint32_t (&a)[N], uint3
     }
 }
 
-template <int N, int I>
+// rows I, I + STEP, ...
+template <int N, int I, int STEP = 1>
 __device__ __forceinline__ void mul_rows(Columns<N>& s, const uint32_t (&a)[N],
                                          const uint32_t (&b)[N])
 {
     if constexpr (I < N) {
         row<N, I, (N - 2 - I > 0 ? N - 2 - I : 0)>(s, a, b[I]);
-        mul_rows<N, I + 1>(s, a, b);
+        mul_rows<N, I + STEP, STEP>(s, a, b);
     }
 }
 
@@ -129,6 +131,29 @@ __device__ __forceinline__ void mul_trunc(const uint32_t (&a)[N], const uint32_t
     clear(s);
     mul_rows<N, 0>(s, a, b);
     add_columns<N>(s, acc);
+}
+
+// The part of mul_trunc's sum from the rows of one parity; the two parts add
+// up to it (add_part).
+template <int N, int PARITY>
+__device__ __forceinline__ void mul_part(const uint32_t (&a)[N], const uint32_t (&b)[N],
+                                         uint32_t (&acc)[N + 2])
+{
+    Columns<N> s;
+    clear(s);
+    mul_rows<N, PARITY, 2>(s, a, b);
+    add_columns<N>(s, acc);
+}
+
+// acc += the words part(0) .. part(N + 1)
+template <int N, class Part>
+__device__ __forceinline__ void add_part(uint32_t (&acc)[N + 2], const Part& part)
+{
+    asm volatile("add.cc.u32 %0, %0, %1;" : "+r"(acc[0]) : "r"(part(0)));
+#pragma unroll
+    for (int k = 1; k < N + 1; ++k)
+        asm volatile("addc.cc.u32 %0, %0, %1;" : "+r"(acc[k]) : "r"(part(k)));
+    asm volatile("addc.u32 %0, %0, %1;" : "+r"(acc[N + 1]) : "r"(part(N + 1)));
 }
 
 // Truncated square of a magnitude; acc as in mul_trunc.

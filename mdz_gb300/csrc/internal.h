@@ -148,8 +148,9 @@ struct MpLaunch {
     const unsigned* list = nullptr;
     const unsigned* list_count = nullptr;
     float* mag = nullptr;   // |z|^2 at escape (FP32), when non-null
-    // lists of at most this many pixels run one pixel a block (set by the launch)
-    unsigned pixel_limit = 0;
+    // lists of at most so many pixels run one pixel a block, four warps for 32
+    // pixels (set by the launch)
+    unsigned pixel_limit = 0, split_limit = 0;
     DoneSignal done;        // optional: stores 1 when the launch is complete
                             // (3 when it also reached the list's end)
     // list pass in chunks: this launch takes tiles tile_base + [0, tile_limit)
@@ -157,16 +158,26 @@ struct MpLaunch {
     // polls a bounded wait of the fused launch makes before it gives up
     int spin_limit = kSpinLimit;
 };
-// Lists of at most this many pixels an SM go to mp_pixel_kernel: a block's
-// iteration takes 0.8 us at N = 8, 0.9 at 16, 1.25 at 34, and each further
-// pixel an SM adds 0.06 to 0.1; a thread's takes 0.47, 1.23, 4.2.  (16000
-// iterations at N = 34, 2.8 pixels an SM: 20.1 ms and 68.2, 8.5: 25.9 and 68.5;
-// 10000 at N = 16, 1.4: 9.1 and 12.5, 5.3: 11.9 and 12.6; at N = 8, 2.6: 12.3
-// and 7.3 for 15000.)
+// Lists of at most this many pixels an SM go to mp_split_kernel, whose
+// iteration of 32 pixels takes 0.51 us at N = 8, 0.60 at 10, 0.93 at 16, 1.44 at
+// 24, 2.25 at 34; a thread's takes 0.48, 0.67, 1.23, 2.3, 4.2.  With more of
+// them the multiplier is full either way.  (Lists at N = 10, 9 pixels an SM:
+// 1.8 ms and 2.0, 38: 2.1 and 2.1; at N = 16, 9: 9.4 and 12.7, 62: 11.7 and 13.4,
+// 80: 13.4 and 13.1; at N = 24, 63: 19.0 and 25.1, 139: 33.8 and 35.5; at N = 34,
+// 62: 37.7 and 69.1.)
+template <int N>
+constexpr int split_list_per_sm()
+{
+    return N >= 16 ? 64 : N >= 10 ? 32 : 0;
+}
+// Of these, lists of at most this many pixels an SM go to mp_pixel_kernel: a
+// block's iteration takes 1.25 us at N = 34, and each further pixel an SM adds
+// 0.06 (16000 iterations, 2.8 pixels an SM: 20.1 ms, 35.6 in mp_split_kernel;
+// 8.5: 25.9 and 36.4); at N = 16 0.9 and 0.06 (2.6 pixels an SM: 9.7 and 9.2).
 template <int N>
 constexpr int pixel_list_per_sm()
 {
-    return N >= 34 ? 32 : N >= 28 ? 18 : N >= 24 ? 10 : N >= 20 ? 7 : N >= 16 ? 5 : 0;
+    return N >= 34 ? 16 : N >= 28 ? 6 : N >= 24 ? 3 : 0;
 }
 int launch_mp(mdzgpu_ctx* ctx, const MpLaunch& p, cudaStream_t s);
 // Kernels launch_mp launches for a list's first chunk.

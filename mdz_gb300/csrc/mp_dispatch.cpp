@@ -42,7 +42,7 @@ int mp_list_launches(int words)
 {
 #define MDZ_CASE(n) \
     if (words == n) \
-        return pixel_list_per_sm<n>() > 0 ? 2 : 1;
+        return 1 + (split_list_per_sm<n>() > 0) + (pixel_list_per_sm<n>() > 0);
     MDZ_MP_WORDS_LIST(MDZ_CASE)
 #undef MDZ_CASE
     return 1;

@@ -168,8 +168,8 @@ __global__ void __launch_bounds__(kFrameBlock, frame_blocks_per_sm<N>())
     const int tiles_y = (p.nrows + kTileH - 1) / kTileH;
     const unsigned list_n = p.list ? *p.list_count : 0u;
     const unsigned listed = (list_n + 31u) / 32u;
-    // (a short list is mp_pixel_kernel's)
-    const unsigned total = p.list ? (list_n <= p.pixel_limit ? 0u : listed)
+    // (a short list is mp_split_kernel's or mp_pixel_kernel's)
+    const unsigned total = p.list ? (list_n <= p.split_limit ? 0u : listed)
                                   : (unsigned)tiles_x * (unsigned)tiles_y;
     unsigned long long its = 0;
     TileFeed feed;
@@ -260,13 +260,176 @@ __global__ void __launch_bounds__(kFrameBlock, frame_blocks_per_sm<N>())
         done_signal(p.done, (unsigned long long)p.tile_base + p.tile_limit >= listed ? 3 : 1);
 }
 
-// ---- short lists: one pixel a block ----
+// ---- short lists: four warps for 32 pixels ----
 //
 // The perturbation hands a few hundred to a few thousand pixels to the
 // multi-limb pass, to run thousands of iterations each; one thread a pixel
 // takes 1.2 us an iteration at N = 16 and 4.2 us at N = 34 however few they
-// are.  Here a block of 4 (N + 1) threads iterates one pixel, with the same
-// truncated products, so the same counts:
+// are.  Here lane i of each of a block's four warps works on the same pixel,
+// with the same truncated products, so the same counts:
+//
+//  1. Warps 0 and 1 form the product wre wim, the even rows and the odd ones;
+//     warps 2 and 3 the squares of wim and wre: N^2 / 4 multiply-adds each.
+//  2. Warp 0 adds the product's halves up to the next wim; warp 3 tests the
+//     squares and goes on to the next wre.
+//
+// What bounds it is latency: each warp's chain of carries, and two barriers an
+// iteration.
+constexpr int kSplitBlock = 128;
+
+template <int N>
+__global__ void __launch_bounds__(kSplitBlock) mp_split_kernel(MpLaunch p, unsigned sms)
+{
+    __shared__ uint32_t zim[N][32], zre[N][32];   // |wim|, |wre| of each lane's pixel
+    __shared__ uint32_t part[N + 2][32];          // the product's odd rows
+    __shared__ uint32_t sq[N][32];                // wim^2
+    __shared__ uint32_t sign_re[32];              // sign mask of wre
+    __shared__ uint32_t top_im[2][32];            // the two top words of wim, signed
+    __shared__ int live;
+    const unsigned list_n = *p.list_count;
+    // a pixel for every block, then a second one, ...: as few blocks an SM as
+    // hold the list
+    const unsigned all = sms * ((list_n + 32u * sms - 1u) / (32u * sms));
+    const unsigned blocks = all < gridDim.x ? all : gridDim.x;
+    if (list_n <= p.pixel_limit || list_n > p.split_limit || blockIdx.x >= blocks
+        || blockIdx.x >= list_n)
+        return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned at = (unsigned)lane * blocks + blockIdx.x;
+    bool done = at >= list_n;
+    const unsigned pix = p.list[done ? blockIdx.x : at];
+    const bool ship = p.fractal == MDZ_BURNING_SHIP;
+    const bool celtic = p.fractal == MDZ_GENERALIZED_CELTIC;
+    const bool variant = p.fractal == MDZ_VARIANT;
+    uint32_t own[N] = {};   // warp 0: |wim|, warp 3: |wre|
+    CRegs<N> c;             // warp 0: c_im, warp 3: c_re
+    uint32_t sign = 0, top1 = 0, top0 = 0;
+    auto publish = [&](uint32_t (*z)[32]) {
+        top1 = own[N - 1];
+        top0 = own[N - 2];
+        sign = fx::abs_inplace<N>(own);
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            z[k][lane] = own[k];
+        if (warp == 0) {
+            top_im[0][lane] = top0;
+            top_im[1][lane] = top1;
+        } else {
+            sign_re[lane] = sign;
+        }
+    };
+    auto start = [&](const uint32_t* z, const uint32_t* julia, uint32_t (*to)[32]) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            own[k] = z[k];
+            c.set(k, p.family == MDZ_FAMILY_JULIA ? julia[k] : own[k]);
+        }
+        publish(to);
+    };
+    const unsigned row = pix / (unsigned)p.W;
+    if (warp == 0)
+        start(p.ys + (size_t)row * N, p.julia + N, zim);
+    else if (warp == 3)
+        start(p.xs + (size_t)(pix - row * (unsigned)p.W) * N, p.julia, zre);
+    auto top_float = [](uint32_t hi, uint32_t lo) {
+        return (float)(int32_t)hi * 5.9604645e-8f /* 2^-24 */
+               + (float)lo * 1.3877788e-17f /* 2^-56 */;
+    };
+    auto big = [](uint32_t hi) {
+        return (int32_t)hi >= 0x08000000 || (int32_t)hi < -0x08000000;
+    };
+    unsigned long long its = 0;
+    if (threadIdx.x == 0)
+        live = 1;
+    __syncthreads();
+    for (uint32_t wz = 0;; ++wz) {
+        uint32_t acc[N + 2], t[N];
+        uint32_t sre = 0;
+        if (warp < 2) {
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                t[k] = zre[k][lane];
+            if (warp == 0) {
+                sre = sign_re[lane];
+                fx::mul_part<N, 0>(t, own, acc);
+            } else {
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    own[k] = zim[k][lane];
+                fx::mul_part<N, 1>(t, own, acc);
+#pragma unroll
+                for (int k = 0; k < N + 2; ++k)
+                    part[k][lane] = acc[k];
+            }
+        } else {
+            if (warp == 2) {
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    own[k] = zim[k][lane];
+            }
+            fx::sqr_trunc<N>(own, acc);
+            fx::extract<N, 24>(acc, t);
+            if (warp == 2) {
+#pragma unroll
+                for (int k = 0; k < N; ++k)
+                    sq[k][lane] = t[k];
+            }
+        }
+        __syncthreads();
+        if (warp == 0) {
+            // wim = 2.0 * wre * wim + c_im   (burning ship: 2 |wre wim| + c_im)
+            fx::add_part<N>(acc, [&](int k) { return part[k][lane]; });
+            fx::extract<N, 23>(acc, t);
+            fx::add_signed<N>(c, t, ship ? 0u : (sre ^ sign), own);
+            publish(zim);
+        } else if (warp == 3) {
+            uint32_t wim2[N], d[N];
+#pragma unroll
+            for (int k = 0; k < N; ++k)
+                wim2[k] = sq[k][lane];
+            if (!done) {
+                const uint32_t im1 = top_im[1][lane], im0 = top_im[0][lane];
+                const bool far = wz && (big(top1) || big(im1));
+                const bool over = far || (wz && fx::sum_gt4<N>(wim2, t));   // not z_0 = c
+                if (over || wz >= p.depth) {
+                    done = true;
+                    float mag;
+                    if (far) {
+                        const float a = top_float(top1, top0), b = top_float(im1, im0);
+                        mag = a * a + b * b;
+                    } else {
+                        mag = fx_top_float<N>(wim2) + fx_top_float<N>(t);
+                    }
+                    p.out[pix] = over ? (int32_t)wz : 0;
+                    if (p.mag)
+                        p.mag[pix] = mag;
+                    its += over ? wz : p.depth;
+                }
+            }
+            // wre = wre2 - wim2 + c_re       (celtic: |wre2 - wim2| + c_re)
+            fx::sub<N>(t, wim2, d);
+            const bool fold = celtic || (variant && !(wz & 1u));
+            fx::add_signed<N>(c, d, fold ? (uint32_t)((int32_t)d[N - 1] >> 31) : 0u, own);
+            const bool any = __any_sync(0xffffffffu, !done);
+            if (lane == 0 && !any)
+                live = 0;
+            publish(zre);
+        }
+        __syncthreads();
+        if (!live)
+            break;
+    }
+    if (warp == 3) {
+        its = warp_sum_u64(its);
+        if (lane == 0)
+            atomicAdd(&p.sync->iter_sum, its);
+    }
+}
+
+// ---- few pixels, many words: a block a pixel ----
+//
+// With a few pixels an SM and 24 words or more, a block of 4 (N + 1) threads
+// iterates one pixel, with the same truncated products again:
 //
 //  1. Thread 4 k + s forms one column sum, column N-2+k, in 96 bits: s = 0, 1
 //     half of the general product's terms each, s = 2, 3 those of the squares
@@ -690,19 +853,29 @@ template <int N>
 int launch_words(mdzgpu_ctx* ctx, const MpLaunch& frame, cudaStream_t s)
 {
     MpLaunch p = frame;
-    p.pixel_limit = 0;
-    if (pixel_list_per_sm<N>() > 0 && p.list && p.tile_base == 0) {
-        // both kernels look at the list's length, which only the device knows,
-        // and one of them leaves; a short list is done in the first chunk (a
-        // later chunk means it was longer than the first one)
-        p.pixel_limit = (unsigned)(pixel_list_per_sm<N>() * ctx->num_sms);
-        constexpr int threads = pixel_threads<N>();
-        int b = 0;
-        if (int rc = pixel_blocks_per_sm<N>(&b))
-            return rc;
-        const long pixels = std::min((long)p.W * p.nrows, (long)p.pixel_limit);
-        mp_pixel_kernel<N><<<(unsigned)std::min(pixels, (long)ctx->num_sms * b), threads, 0, s>>>(p);
-        MDZ_CUDA_TRY(cudaGetLastError());
+    p.pixel_limit = p.split_limit = 0;
+    // The kernels look at the list's length, which only the device knows, and
+    // all but one of them leave; a short list is done in the first chunk (a
+    // later chunk means it was longer than the first one).
+    if constexpr (split_list_per_sm<N>() > 0) {
+        if (p.list && p.tile_base == 0) {
+            p.pixel_limit = (unsigned)(pixel_list_per_sm<N>() * ctx->num_sms);
+            p.split_limit = (unsigned)(split_list_per_sm<N>() * ctx->num_sms);
+            if constexpr (pixel_list_per_sm<N>() > 0) {
+                constexpr int threads = pixel_threads<N>();
+                int b = 0;
+                if (int rc = pixel_blocks_per_sm<N>(&b))
+                    return rc;
+                const long pixels = std::min((long)p.W * p.nrows, (long)p.pixel_limit);
+                mp_pixel_kernel<N>
+                    <<<(unsigned)std::min(pixels, (long)ctx->num_sms * b), threads, 0, s>>>(p);
+                MDZ_CUDA_TRY(cudaGetLastError());
+            }
+            // (32 pixels a block; the blocks do not wait for one another)
+            mp_split_kernel<N><<<(unsigned)(split_list_per_sm<N>() / 32 * ctx->num_sms),
+                                 kSplitBlock, 0, s>>>(p, (unsigned)ctx->num_sms);
+            MDZ_CUDA_TRY(cudaGetLastError());
+        }
     }
     const bool julia = p.family == MDZ_FAMILY_JULIA;
     switch (p.fractal) {
@@ -746,7 +919,14 @@ int launch_serve_mp_words(ServeDev* d, int mp_class, int num_sms, cudaStream_t s
 template <int N>
 int preload_words()
 {
-    int b = 0, rc = pixel_blocks_per_sm<N>(&b);
+    int b = 0, rc = MDZGPU_OK;
+    if constexpr (pixel_list_per_sm<N>() > 0)
+        rc = pixel_blocks_per_sm<N>(&b);
+    if constexpr (split_list_per_sm<N>() > 0) {
+        if (!rc)
+            MDZ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, mp_split_kernel<N>,
+                                                                       kSplitBlock, 0));
+    }
     for (int j = 0; j < 2 && !rc; ++j) {
         const bool julia = j == 1;
         rc = julia ? typed_blocks_per_sm<N, MDZ_MANDELBROT, true>(&b)
