@@ -33,6 +33,7 @@ namespace {
 
 constexpr int kRefill = 4;        // idle lanes that make a warp take new pixels
 constexpr int kRefillEvery = 8;   // iterations between looks at the idle lanes
+constexpr int kLookEvery = 8;     // these between looks at the block's other warps
 
 template <int N>
 struct CRegs {
@@ -143,25 +144,27 @@ __host__ __device__ constexpr int block_threads()
     return N > 16 ? 128 : 256;
 }
 
-// Frame launches take blocks of four warps, one for each of an SM's schedulers,
-// so that a frame or list of few tiles spreads over all SMs (blocks of eight
-// left the 949 tiles of a 201x151 frame at N = 34 70 to 86 ms, against 66),
-// and at most 16 warps an SM: with 24 nothing gains (640x480-class frames at
-// 4 and 10 words, within 3%), with 8 the multiplier waits (27 -> 29 ms).
-constexpr int kFrameBlock = 128;
-
+// A frame launch takes one block an SM, whose warps merge as pixels finish
+// (pixel_feed.cuh): at most 16 warps (with 24 nothing gains, with 8 the
+// multiplier waits: 640x480-class frames at 4 and 10 words).
 template <int N>
-__host__ __device__ constexpr int frame_blocks_per_sm()
+__host__ __device__ constexpr int frame_block()
 {
-    return N > 20 ? 2 : N > 16 ? 3 : 4;
+    return N > 20 ? 256 : N > 16 ? 384 : 512;
 }
+constexpr int kFrameMove = 64;   // pixels moved to other warps at a time
 
 template <int N, int FRACTAL, bool JULIA>
-__global__ void __launch_bounds__(kFrameBlock, frame_blocks_per_sm<N>())
-    mp_frame_kernel(MpLaunch p)
+__global__ void __launch_bounds__(frame_block<N>(), 1) mp_frame_kernel(MpLaunch p)
 {
     extern __shared__ uint32_t smem[];
-    __shared__ int2 tile[kFrameBlock / 32][32];   // the warp's current tile
+    constexpr int kBlock = frame_block<N>(), kWarps = kBlock / 32;
+    __shared__ int2 tile[kWarps][32];   // the warp's current tile
+    __shared__ LaneMerge<kWarps> merge;
+    __shared__ uint32_t moved[2 * N + 5][kFrameMove];
+    merge.init();
+    int kept = kWarps;
+    bool dry = false;   // the tiles are used up
     using CGet = typename std::conditional<c_in_smem<N>(), CShared<N>, CRegs<N>>::type;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tiles_x = (p.W + kTileW - 1) / kTileW;
@@ -179,12 +182,42 @@ __global__ void __launch_bounds__(kFrameBlock, frame_blocks_per_sm<N>())
     MpOrbit<N> o;
     CGet c_re, c_im;
     if constexpr (c_in_smem<N>()) {
-        c_re = CGet{smem + threadIdx.x, kFrameBlock};
-        c_im = CGet{smem + N * kFrameBlock + threadIdx.x, kFrameBlock};
+        c_re = CGet{smem + threadIdx.x, kBlock};
+        c_im = CGet{smem + N * kBlock + threadIdx.x, kBlock};
     }
     for (;;) {
         if (p.tile_rows_done && !p.list)
             count_bands(p.W, p.nrows, p.tile_rows_done, p.band_flags, band);
+        bool came = false;   // from another warp
+        if (dry && merge.look(feed, active, kept)
+            && !merge.merge(
+                feed, active, kept, kFrameMove,
+                [&](int k) {
+#pragma unroll
+                    for (int j = 0; j < N; ++j) {
+                        moved[j][k] = o.wre[j];
+                        moved[N + j][k] = o.wim[j];
+                    }
+                    moved[2 * N][k] = o.sre;
+                    moved[2 * N + 1][k] = o.sim;
+                    moved[2 * N + 2][k] = o.wz;
+                    moved[2 * N + 3][k] = (uint32_t)ix;
+                    moved[2 * N + 4][k] = (uint32_t)lrow;
+                },
+                [&](int k) {
+#pragma unroll
+                    for (int j = 0; j < N; ++j) {
+                        o.wre[j] = moved[j][k];
+                        o.wim[j] = moved[N + j][k];
+                    }
+                    o.sre = moved[2 * N][k];
+                    o.sim = moved[2 * N + 1][k];
+                    o.wz = moved[2 * N + 2][k];
+                    ix = (int)moved[2 * N + 3][k];
+                    lrow = (int)moved[2 * N + 4][k];
+                    came = true;
+                }))
+            break;
         bool fresh = false;
         feed_lanes(
             feed, !active,
@@ -211,23 +244,38 @@ __global__ void __launch_bounds__(kFrameBlock, frame_blocks_per_sm<N>())
                 lrow = tile[warp][k].y;
                 fresh = true;
             });
-        if (fresh) {
+        if (fresh || came) {
             const uint32_t* xs = p.xs + (size_t)ix * N;
             const uint32_t* ys = p.ys + (size_t)lrow * N;
 #pragma unroll
             for (int k = 0; k < N; ++k) {
-                o.wre[k] = xs[k];
-                o.wim[k] = ys[k];
-                c_re.set(k, JULIA ? p.julia[k] : o.wre[k]);
-                c_im.set(k, JULIA ? p.julia[N + k] : o.wim[k]);
+                const uint32_t x = xs[k], y = ys[k];
+                if (fresh) {
+                    o.wre[k] = x;
+                    o.wim[k] = y;
+                }
+                c_re.set(k, JULIA ? p.julia[k] : x);
+                c_im.set(k, JULIA ? p.julia[N + k] : y);
             }
-            mp_start<N>(o);
+            if (fresh) {
+                o.sre = fx::abs_inplace<N>(o.wre);
+                o.sim = fx::abs_inplace<N>(o.wim);
+                o.wz = 0;
+            }
+            float mag;
+            mp_squares<N>(o, false, mag);   // z_0 = c is not tested
             active = true;
         }
+        if (!feed.left && !feed.more && !dry) {
+            dry = true;
+            if (lane == 0)
+                merge.set_dry();
+        }
         if (!__any_sync(0xffffffffu, active))
-            break;
+            continue;
         // iterate until enough lanes are idle to be worth a look
         const int enough = (feed.left || feed.more) ? kRefill : 32;
+        int looks = kLookEvery;
         do {
             if (active) {
                 int u = kRefillEvery;
@@ -251,6 +299,13 @@ __global__ void __launch_bounds__(kFrameBlock, frame_blocks_per_sm<N>())
                     band = lrow / kTileH;
                 }
             }
+            if (!dry && merge.is_dry()) {
+                dry = true;
+                feed.more = false;
+                break;
+            }
+            if (dry && --looks == 0)
+                break;
         } while (__popc(__ballot_sync(0xffffffffu, !active)) < enough);
     }
     its = warp_sum_u64(its);
@@ -794,18 +849,18 @@ __global__ void __launch_bounds__(block_threads<N>()) serve_mp_kernel(ServeDev* 
 template <int N, int FRACTAL, bool JULIA>
 int typed_blocks_per_sm(int* out)
 {
-    constexpr int threads = kFrameBlock;
+    constexpr int threads = frame_block<N>();
     const size_t smem = c_in_smem<N>() ? (size_t)2 * N * threads * sizeof(uint32_t) : 0;
     static int blocks_per_sm = 0;
     if (!blocks_per_sm) {
-        if (smem > 48 * 1024)
+        if (smem)   // beside the static part
             MDZ_CUDA_TRY(cudaFuncSetAttribute(mp_frame_kernel<N, FRACTAL, JULIA>,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)smem));
         int b = 0;
         MDZ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
             &b, mp_frame_kernel<N, FRACTAL, JULIA>, threads, smem));
-        blocks_per_sm = b < 1 ? 1 : (b < frame_blocks_per_sm<N>() ? b : frame_blocks_per_sm<N>());
+        blocks_per_sm = 1;
     }
     *out = blocks_per_sm;
     return MDZGPU_OK;
@@ -828,7 +883,7 @@ int pixel_blocks_per_sm(int* out)
 template <int N, int FRACTAL, bool JULIA>
 int launch_typed(mdzgpu_ctx* ctx, const MpLaunch& p, cudaStream_t s)
 {
-    constexpr int threads = kFrameBlock;
+    constexpr int threads = frame_block<N>();
     const size_t smem = c_in_smem<N>() ? (size_t)2 * N * threads * sizeof(uint32_t) : 0;
     int blocks_per_sm = 1;
     if (int rc = typed_blocks_per_sm<N, FRACTAL, JULIA>(&blocks_per_sm))
