@@ -51,10 +51,11 @@ VIEWS = json.loads((ROOT / "tests" / "golden" / "views.json").read_text())
 # (8 flops); the roofline counts the algorithmic 16 against the FP32 flop
 # peak (2 flops per FFMA lane).
 ALGO_OPS_PER_PIXEL_ITER = 16
-# DRAM bytes (read + written) of one perturb_step_kernel launch of the
-# 1920x1080 2^-1000 frame: ncu dram__bytes_read.sum + dram__bytes_write.sum
-# (one pass, --clock-control none) over launches 61-63 of one frame, 74.7 MB
-# read and 11.6-14.6 MB written each (profiles/perturb_step_kernel_c4_traffic.md).
+# DRAM bytes (read + written) of one pixel-step launch of the 1920x1080
+# 2^-1000 frame: ncu dram__bytes_read.sum + dram__bytes_write.sum (one pass,
+# --clock-control none) over launches 61-63 of one frame, 74.7 MB read and
+# 11.6-14.6 MB written each, taken with one pixel a lane
+# (profiles/perturb_step_kernel_c4_traffic.md); two a lane move the same state.
 # The pixel state (32 B per unfinished pixel) goes in and out once a launch;
 # the reference orbit (3.2 MB of float4 entries) is read from L2.
 STEP_LAUNCH_DRAM_BYTES = 87.6e6
@@ -497,7 +498,7 @@ def run_ours(args, view, world, rank, local, dist):
         r.close()
         return
     ms_per_step = total_ms_max / args.steps
-    # the dominant kernel is the FP32 pixel pass (perturb_step_kernel, one
+    # the dominant kernel is the FP32 pixel pass (perturb_pairs_kernel, one
     # launch per step of the frame): its device time is the sum of CUDA-event
     # intervals around each launch, on the stream it runs on
     avg_pixel_ms = sum(pixel_ms) / len(pixel_ms)
@@ -521,7 +522,7 @@ def run_ours(args, view, world, rank, local, dist):
         "rebases_per_step": rebases / args.steps,
         "e2e": {"value": e2e_its_all / (e2e_max * 1e-3), "unit": "pixel-iters/s",
                 "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-        "roofline": {"bound": "fp32-pipe", "kernel": "perturb_step_kernel",
+        "roofline": {"bound": "fp32-pipe", "kernel": "perturb_pairs_kernel",
                      "achieved": achieved, "peak": peak_gflops,
                      "unit": "GFLOP/s", "frac": achieved / peak_gflops,
                      "algorithmic_flops_per_pixel_iter": ALGO_OPS_PER_PIXEL_ITER,

@@ -308,7 +308,7 @@ struct PerturbLaunch {
 int launch_perturb(mdzgpu_ctx* ctx, const PerturbLaunch& p, cudaStream_t s, int pass);
 // The orbit as a cooperative producer + finisher launch that publishes its
 // progress: progress[1] digits written, [2] entries finished (in whole
-// batches of 256), [3] producer done (final length in *o.out_len), [4] a
+// batches of its block size), [3] producer done (final length in *o.out_len), [4] a
 // bounded wait gave up, [5] SM id + 1 of the producer while it runs.
 // `done` (optional) stores 1 when the launch is complete, 2 if it gave up.
 int launch_orbit_stream(const OrbitLaunch& o, int* progress, cudaStream_t s,
@@ -319,13 +319,13 @@ int launch_orbit_stream(const OrbitLaunch& o, int* progress, cudaStream_t s,
 // unfinished ones go to out; counters[0] = pull counter, counters[1] = out
 // count, counters[2] = working blocks (all reset by the launch).  Blocks
 // placed on the orbit producer's SM (p.producer_sm) leave it to the producer.
-// Whether a step over n pixels takes two a lane (perturb_pairs_kernel): where
-// the deltas start below the FP32 range and every warp of the chip gets 64.
-bool perturb_in_pairs(int num_sms, const PerturbLaunch& p, size_t n);
 int launch_perturb_step(int num_sms, const PerturbLaunch& p, const unsigned* in, unsigned n,
                         unsigned* out, unsigned* counters, uint4* state, unsigned budget,
                         cudaStream_t s, cudaEvent_t before = nullptr,
                         cudaEvent_t after = nullptr);
+// Whether a step over n pixels takes two a lane (perturb_pairs_kernel): where
+// the deltas start below the FP32 range and every warp of the chip gets 64.
+bool perturb_in_pairs(int num_sms, const PerturbLaunch& p, size_t n);
 // Orbit + FP32 pixel pass in one cooperative launch (progress words in p).
 int launch_fused(mdzgpu_ctx* ctx, const OrbitLaunch& o, const PerturbLaunch& p, cudaStream_t s);
 

@@ -145,8 +145,10 @@ __host__ __device__ constexpr int block_threads()
 }
 
 // A frame launch takes one block an SM, whose warps merge as pixels finish
-// (pixel_feed.cuh): at most 16 warps (with 24 nothing gains, with 8 the
-// multiplier waits: 640x480-class frames at 4 and 10 words).
+// (pixel_feed.cuh): 320x240 at 80 bits, counts 0.70 of the depth on average,
+// 8.08 ms in four blocks of four warps an SM, 6.8 in one of 16.  At most 16
+// warps (with 24 nothing gains, with 8 the multiplier waits: 640x480-class
+// frames at 4 and 10 words).
 template <int N>
 __host__ __device__ constexpr int frame_block()
 {
