@@ -330,6 +330,10 @@ __global__ void __launch_bounds__(frame_block<N>(), 1) mp_frame_kernel(MpLaunch 
 //  2. Warp 0 adds the product's halves up to the next wim; warp 3 tests the
 //     squares and goes on to the next wre.
 //
+// A barrier ends each step, and no array is read and written in the same one:
+// z and what goes with it are read in 1 and written in 2, the products' parts
+// the other way round.
+//
 // What bounds it is latency: each warp's chain of carries, and two barriers an
 // iteration.
 constexpr int kSplitBlock = 128;
@@ -401,7 +405,7 @@ __global__ void __launch_bounds__(kSplitBlock) mp_split_kernel(MpLaunch p, unsig
     __syncthreads();
     for (uint32_t wz = 0;; ++wz) {
         uint32_t acc[N + 2], t[N];
-        uint32_t sre = 0;
+        uint32_t sre = 0, im1 = 0, im0 = 0;
         if (warp < 2) {
 #pragma unroll
             for (int k = 0; k < N; ++k)
@@ -423,6 +427,10 @@ __global__ void __launch_bounds__(kSplitBlock) mp_split_kernel(MpLaunch p, unsig
 #pragma unroll
                 for (int k = 0; k < N; ++k)
                     own[k] = zim[k][lane];
+            } else {
+                // before the barrier: past it warp 0 puts the next z's there
+                im1 = top_im[1][lane];
+                im0 = top_im[0][lane];
             }
             fx::sqr_trunc<N>(own, acc);
             fx::extract<N, 24>(acc, t);
@@ -445,7 +453,6 @@ __global__ void __launch_bounds__(kSplitBlock) mp_split_kernel(MpLaunch p, unsig
             for (int k = 0; k < N; ++k)
                 wim2[k] = sq[k][lane];
             if (!done) {
-                const uint32_t im1 = top_im[1][lane], im0 = top_im[0][lane];
                 const bool far = wz && (big(top1) || big(im1));
                 const bool over = far || (wz && fx::sum_gt4<N>(wim2, t));   // not z_0 = c
                 if (over || wz >= p.depth) {
