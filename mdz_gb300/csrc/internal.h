@@ -117,7 +117,7 @@ struct Fp64Launch {
     int W, H;           // real frame size
     int row0, nrows;    // rows rendered by this launch
     int family, fractal;
-    uint32_t depth;
+    uint32_t depth;     // 1 .. INT32_MAX
     double xmin, xmax, ymax, jre, jim;
     int32_t* out;       // out[(line - row0) * W + ix]
     FrameSync* sync;
@@ -133,7 +133,7 @@ int launch_fp64(mdzgpu_ctx* ctx, const Fp64Launch& p, cudaStream_t s);
 struct MpLaunch {
     int W, H, row0, nrows;
     int family, fractal;
-    uint32_t depth;
+    uint32_t depth;          // 1 .. INT32_MAX
     int words;               // 32-bit words per fixed-point number
     const uint32_t* xs;      // [W][words] pixel x coordinates
     const uint32_t* ys;      // [nrows][words] pixel y coordinates
@@ -254,7 +254,7 @@ int orbit_max_limbs();
 
 struct PerturbLaunch {
     int W, H, row0, nrows;
-    uint32_t depth;
+    uint32_t depth;     // 1 .. INT32_MAX
     // Julia family (q_len non-null): entries [0, *orbit_len) are the view
     // orbit V (V_0 = centre, no dc term: a pixel starts at V_0 with its
     // offset as delta); entries [q0, q0 + *q_len) the critical orbit Q

@@ -128,6 +128,14 @@ mdzgpu_mpval as_mpval(const mdz_mpfr* v)
     return m;
 }
 
+// The reference iterates for wz = 1 .. depth, and its counts are ints.  The
+// kernels take depths from 1 on (they test the depth after an iteration);
+// below that every count is 0 and nothing is launched.
+uint32_t image_depth(const mdz_image_info* img)
+{
+    return (uint32_t)(img->depth < 0 ? 0 : img->depth > 0x7fffffff ? 0x7fffffff : img->depth);
+}
+
 // Fixed-point tables for rows [row0, row0 + nrows): x[W] | y[nrows] |
 // julia c_re | c_im.  MPFR callback: MPFR's own p-bit coordinate roundings
 // (src/fractal.c:159-203).  GMP callback: exact values from gxmin / gymax /
@@ -203,6 +211,7 @@ int gpu_frame(mdz_rthdata* rth, Method method)
     }
     const int nbands = (H + 3) / 4;
     const size_t n = (size_t)W * H;
+    const uint32_t depth = image_depth(img);
     int rc = ctx->staging.ensure(n * sizeof(int32_t));
     if (!rc)
         rc = ctx->pinned.ensure((size_t)(nbands + 64) * sizeof(int));
@@ -236,7 +245,7 @@ int gpu_frame(mdz_rthdata* rth, Method method)
         p.nrows = H;
         p.family = img->family;
         p.fractal = img->fractal;
-        p.depth = (uint32_t)(img->depth > 0x7fffffff ? 0x7fffffff : img->depth);
+        p.depth = depth;
         // src/fractal.c:50-58: mpfr_get_ld(..., GMP_RNDN), long double = double
         p.xmin = mpfr_to_double_rn(img->xmin);
         p.xmax = mpfr_to_double_rn(img->xmax);
@@ -248,7 +257,7 @@ int gpu_frame(mdz_rthdata* rth, Method method)
         p.tile_rows_done = dbands;
         p.band_flags = dflags;
         p.stop = dstop;
-        rc = launch_fp64(ctx, p, s);
+        rc = depth ? launch_fp64(ctx, p, s) : 0;
     } else {
         const int words_req = mp_words_for_precision(img->precision);
         int words = -1;
@@ -282,7 +291,7 @@ int gpu_frame(mdz_rthdata* rth, Method method)
         p.nrows = H;
         p.family = img->family;
         p.fractal = img->fractal;
-        p.depth = (uint32_t)(img->depth > 0x7fffffff ? 0x7fffffff : img->depth);
+        p.depth = depth;
         p.words = words;
         p.xs = (const uint32_t*)ctx->coords.ptr;
         p.ys = p.xs + (size_t)W * words;
@@ -292,7 +301,12 @@ int gpu_frame(mdz_rthdata* rth, Method method)
         p.tile_rows_done = dbands;
         p.band_flags = dflags;
         p.stop = dstop;
-        rc = launch_mp(ctx, p, s);
+        rc = depth ? launch_mp(ctx, p, s) : 0;
+    }
+    if (!depth) {
+        memset(ctx->staging.host, 0, n * sizeof(int32_t));
+        for (int b = 0; b < nbands; ++b)
+            hflags[b] = 1;
     }
     cudaEvent_t done_ev;
     if (rc || cudaEventCreateWithFlags(&done_ev, cudaEventDisableTiming) != cudaSuccess) {
@@ -461,6 +475,7 @@ int line_render(mdz_image_info* img, int line, Method method)
     const int W = img->real_width;
     if (line < 0 || line >= img->real_height)
         return 0;
+    const uint32_t depth = image_depth(img);
     int rc = ctx->counts.ensure((size_t)W * sizeof(int32_t));
     if (!rc)
         rc = ctx->sync.ensure(sizeof(FrameSync));
@@ -476,7 +491,7 @@ int line_render(mdz_image_info* img, int line, Method method)
         p.nrows = 1;
         p.family = img->family;
         p.fractal = img->fractal;
-        p.depth = (uint32_t)img->depth;
+        p.depth = depth;
         p.xmin = mpfr_to_double_rn(img->xmin);
         p.xmax = mpfr_to_double_rn(img->xmax);
         p.ymax = mpfr_to_double_rn(img->ymax);
@@ -487,7 +502,7 @@ int line_render(mdz_image_info* img, int line, Method method)
         p.tile_rows_done = nullptr;
         p.band_flags = nullptr;
         p.stop = nullptr;
-        if (launch_fp64(ctx, p, ctx->stream))
+        if (depth && launch_fp64(ctx, p, ctx->stream))
             return 0;
     } else {
         int words = -1;
@@ -512,7 +527,7 @@ int line_render(mdz_image_info* img, int line, Method method)
         p.nrows = 1;
         p.family = img->family;
         p.fractal = img->fractal;
-        p.depth = (uint32_t)img->depth;
+        p.depth = depth;
         p.words = words;
         p.xs = (const uint32_t*)ctx->coords.ptr;
         p.ys = p.xs + (size_t)W * words;
@@ -522,9 +537,11 @@ int line_render(mdz_image_info* img, int line, Method method)
         p.tile_rows_done = nullptr;
         p.band_flags = nullptr;
         p.stop = nullptr;
-        if (launch_mp(ctx, p, ctx->stream))
+        if (depth && launch_mp(ctx, p, ctx->stream))
             return 0;
     }
+    if (!depth)
+        cudaMemsetAsync(ctx->counts.ptr, 0, (size_t)W * 4, ctx->stream);
     if (cudaMemcpyAsync(img->raw_data + (size_t)line * W, ctx->counts.ptr, (size_t)W * 4,
                         cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess
         || cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
