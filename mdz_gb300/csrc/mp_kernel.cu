@@ -852,27 +852,34 @@ __global__ void __launch_bounds__(block_threads<N>()) serve_mp_kernel(ServeDev* 
     }
 }
 
-// Attributes and occupancy of one frame kernel, set up once.  The first
-// call also loads the kernel (with lazy module loading, a load waits for
-// the work running on the device, so servers call it before they start).
-template <int N, int FRACTAL, bool JULIA>
-int typed_blocks_per_sm(int* out)
+// Dynamic shared memory of a frame block: c, above 16 words.
+template <int N>
+constexpr size_t frame_smem()
 {
-    constexpr int threads = frame_block<N>();
-    const size_t smem = c_in_smem<N>() ? (size_t)2 * N * threads * sizeof(uint32_t) : 0;
-    static int blocks_per_sm = 0;
-    if (!blocks_per_sm) {
-        if (smem)   // beside the static part
-            MDZ_CUDA_TRY(cudaFuncSetAttribute(mp_frame_kernel<N, FRACTAL, JULIA>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)smem));
-        int b = 0;
-        MDZ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &b, mp_frame_kernel<N, FRACTAL, JULIA>, threads, smem));
-        blocks_per_sm = 1;
-    }
-    *out = blocks_per_sm;
+    return c_in_smem<N>() ? (size_t)2 * N * frame_block<N>() * sizeof(uint32_t) : 0;
+}
+
+// Lets a frame kernel have its shared memory (with the static part it passes
+// the 48 KB that need no leave from 20 words on).  The leave is the current
+// device's, so every launch asks: a process may render on several.
+template <int N, int FRACTAL, bool JULIA>
+int allow_frame_smem()
+{
+    if (frame_smem<N>())
+        MDZ_CUDA_TRY(cudaFuncSetAttribute(mp_frame_kernel<N, FRACTAL, JULIA>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)frame_smem<N>()));
     return MDZGPU_OK;
+}
+
+// Loads one frame kernel: with lazy module loading, a load waits for the work
+// running on the device, so servers call it before they start.
+template <int N, int FRACTAL, bool JULIA>
+int load_frame_kernel()
+{
+    cudaFuncAttributes a;
+    MDZ_CUDA_TRY(cudaFuncGetAttributes(&a, mp_frame_kernel<N, FRACTAL, JULIA>));
+    return allow_frame_smem<N, FRACTAL, JULIA>();
 }
 
 template <int N>
@@ -893,20 +900,18 @@ template <int N, int FRACTAL, bool JULIA>
 int launch_typed(mdzgpu_ctx* ctx, const MpLaunch& p, cudaStream_t s)
 {
     constexpr int threads = frame_block<N>();
-    const size_t smem = c_in_smem<N>() ? (size_t)2 * N * threads * sizeof(uint32_t) : 0;
-    int blocks_per_sm = 1;
-    if (int rc = typed_blocks_per_sm<N, FRACTAL, JULIA>(&blocks_per_sm))
+    if (int rc = allow_frame_smem<N, FRACTAL, JULIA>())
         return rc;
     const long tiles = p.list ? ((long)p.W * p.nrows + 31) / 32
                               : (long)((p.W + kTileW - 1) / kTileW) * ((p.nrows + kTileH - 1) / kTileH);
-    long grid = (long)ctx->num_sms * blocks_per_sm;
+    long grid = ctx->num_sms;   // a block an SM
     const long blocks_needed = std::max((tiles + threads / 32 - 1) / (threads / 32),
                                         std::min(tiles, (long)ctx->num_sms));
     if (grid > blocks_needed)
         grid = blocks_needed;
     if (grid < 1)
         grid = 1;
-    mp_frame_kernel<N, FRACTAL, JULIA><<<(unsigned)grid, threads, smem, s>>>(p);
+    mp_frame_kernel<N, FRACTAL, JULIA><<<(unsigned)grid, threads, frame_smem<N>(), s>>>(p);
     MDZ_CUDA_TRY(cudaGetLastError());
     return MDZGPU_OK;
 }
@@ -993,17 +998,17 @@ int preload_words()
     }
     for (int j = 0; j < 2 && !rc; ++j) {
         const bool julia = j == 1;
-        rc = julia ? typed_blocks_per_sm<N, MDZ_MANDELBROT, true>(&b)
-                   : typed_blocks_per_sm<N, MDZ_MANDELBROT, false>(&b);
+        rc = julia ? load_frame_kernel<N, MDZ_MANDELBROT, true>()
+                   : load_frame_kernel<N, MDZ_MANDELBROT, false>();
         if (!rc)
-            rc = julia ? typed_blocks_per_sm<N, MDZ_BURNING_SHIP, true>(&b)
-                       : typed_blocks_per_sm<N, MDZ_BURNING_SHIP, false>(&b);
+            rc = julia ? load_frame_kernel<N, MDZ_BURNING_SHIP, true>()
+                       : load_frame_kernel<N, MDZ_BURNING_SHIP, false>();
         if (!rc)
-            rc = julia ? typed_blocks_per_sm<N, MDZ_GENERALIZED_CELTIC, true>(&b)
-                       : typed_blocks_per_sm<N, MDZ_GENERALIZED_CELTIC, false>(&b);
+            rc = julia ? load_frame_kernel<N, MDZ_GENERALIZED_CELTIC, true>()
+                       : load_frame_kernel<N, MDZ_GENERALIZED_CELTIC, false>();
         if (!rc)
-            rc = julia ? typed_blocks_per_sm<N, MDZ_VARIANT, true>(&b)
-                       : typed_blocks_per_sm<N, MDZ_VARIANT, false>(&b);
+            rc = julia ? load_frame_kernel<N, MDZ_VARIANT, true>()
+                       : load_frame_kernel<N, MDZ_VARIANT, false>();
     }
     return rc;
 }
