@@ -238,6 +238,17 @@ int mdzgpu_set_wait_limit(mdzgpu_ctx* ctx, int32_t polls);
 int mdzgpu_last_escalations(mdzgpu_ctx* ctx, uint32_t* fp64, int64_t cap_fp64, int64_t* n_fp64,
                             uint32_t* mp, int64_t cap_mp, int64_t* n_mp);
 
+/* No counterpart in the reference.  The fixed-point digits of a reference
+ * orbit of the last perturbation render on this context (which = 0: the orbit,
+ * the Julia family's view orbit, the hybrid's that folds at odd steps; 1: the
+ * second one of these two).  Entry k holds *limbs real and *limbs imaginary
+ * digits, lowest first, Z_k = sum d_j 2^(28 (j - *limbs + 1)).  Copies at most
+ * `capacity` entries; *len receives their number.  Valid until the context's
+ * next perturbation render or reference orbit; MDZGPU_ERR_ARG when there is
+ * none. */
+int mdzgpu_last_orbit_digits(mdzgpu_ctx* ctx, int32_t which, int32_t* digits, int64_t capacity,
+                             int32_t* limbs, int64_t* len);
+
 /* Largest `words` value the MP kernel is built for. */
 int32_t mdzgpu_mp_max_words(void);
 

@@ -771,6 +771,7 @@ static int perturb_common(mdzgpu_ctx* ctx, const mdzgpu_frame* f, const mdzgpu_m
     const size_t off_zd = ol.zd, off_ze = ol.ze, off_dd = ol.dd, off_de = ol.de;
     const size_t off_len = ol.len, off_dig = ol.bytes, off_reb = ol.reb, off_raw = ol.raw;
     const size_t orbit_bytes = ol.bytes + dig.size() * sizeof(int);
+    ctx->orbit_limbs = 0;
     if ((rc = ctx->orbit.ensure(orbit_bytes)) || (rc = ctx->sync.ensure(sizeof(FrameSync))))
         return rc;
     if (!d_out) {
@@ -1057,8 +1058,13 @@ static int perturb_common(mdzgpu_ctx* ctx, const mdzgpu_frame* f, const mdzgpu_m
         st->esc_fp64_ms = e64;
         st->esc_mp_ms = mp_skipped ? 0.0 : emp;
     }
-    if (!rc)
+    if (!rc) {
         ctx->esc_pixels = (int64_t)n;
+        ctx->orbit_limbs = L;
+        ctx->orbit_digits = off_raw;
+        ctx->orbit_len = off_len;
+        ctx->orbit_second = q0;
+    }
     cudaEventDestroy(evo);
     return rc;
 }
@@ -1088,6 +1094,36 @@ int mdzgpu_last_escalations(mdzgpu_ctx* ctx, uint32_t* fp64, int64_t cap_fp64, i
     MDZ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     *n_fp64 = cnt[0];
     *n_mp = cnt[1];
+    return MDZGPU_OK;
+}
+
+int mdzgpu_last_orbit_digits(mdzgpu_ctx* ctx, int32_t which, int32_t* digits, int64_t capacity,
+                             int32_t* limbs, int64_t* len)
+{
+    if (!ctx || !limbs || !len || capacity < 0 || (capacity && !digits)) {
+        set_error("orbit digits: null argument or negative capacity");
+        return MDZGPU_ERR_ARG;
+    }
+    if (!ctx->orbit_limbs || which < 0 || which > (ctx->orbit_second ? 1 : 0)) {
+        set_error("orbit digits: no such orbit on this context");
+        return MDZGPU_ERR_ARG;
+    }
+    const char* ob = (const char*)ctx->orbit.ptr;
+    int n = 0;
+    MDZ_CUDA_TRY(cudaMemcpyAsync(&n, ob + ctx->orbit_len + (which ? 16 * sizeof(int) : 0), 4,
+                                 cudaMemcpyDeviceToHost, ctx->stream));
+    MDZ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    const size_t entry = 2 * sizeof(int) * (size_t)ctx->orbit_limbs;
+    const int64_t copied = std::min<int64_t>(n, capacity);
+    if (copied)
+        MDZ_CUDA_TRY(cudaMemcpyAsync(digits,
+                                     ob + ctx->orbit_digits
+                                         + (which ? ctx->orbit_second * entry : 0),
+                                     (size_t)copied * entry, cudaMemcpyDeviceToHost,
+                                     ctx->stream));
+    MDZ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    *limbs = ctx->orbit_limbs;
+    *len = n;
     return MDZGPU_OK;
 }
 
@@ -1133,6 +1169,7 @@ int mdzgpu_reference_orbit_formula(mdzgpu_ctx* ctx, int32_t fractal, const mdzgp
     const size_t off_dig = off_len + 256;
     const size_t off_raw = off_dig + al(2 * L * sizeof(int));
     const size_t bytes = off_raw + al(entries * 2 * (size_t)L * sizeof(int));
+    ctx->orbit_limbs = 0;
     int rc = ctx->orbit.ensure(bytes);
     if (rc)
         return rc;

@@ -105,6 +105,11 @@ struct mdzgpu_ctx {
     // pixels of the last perturbation render (its escalation lists sit in
     // `lists`); 0 when no list is current
     int64_t esc_pixels = 0;
+    // the last perturbation render's orbits in `orbit`: digits per number (0:
+    // none current), offsets of the digits and of the first one's length, and
+    // the second one's first entry (0: one orbit)
+    int orbit_limbs = 0;
+    size_t orbit_digits = 0, orbit_len = 0, orbit_second = 0;
 };
 
 namespace mdz {

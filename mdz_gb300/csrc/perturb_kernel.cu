@@ -404,7 +404,8 @@ __device__ __forceinline__ int low_digit(unsigned v)
 // + f 2^28, the first pass leaves t + f' 2^28 (t = d + e', primes: the column
 // below), so the second needs only d, e of the column below and e, f of the
 // one below that: one round of shuffles.  A warp's lowest two columns get no
-// right digits (they are the warp below's; warp 0's lowest is zero).
+// right digits: no lane below them holds what they need.  They are the warp
+// below's, or warp 0's empty column and the lowest one kept.
 __device__ __forceinline__ int carried_digit(long long v)
 {
     const int d = low_digit((unsigned)v);
@@ -557,8 +558,10 @@ __device__ __forceinline__ void orbit_produce_lean(const OrbitLaunch& p, const O
             // digits' most significant nonzero one
             const bool re_part = part == 0;
             d = carried_digit(re_part ? v : v + cc);
+            // (the lowest column of all takes no carry, and carried_digit's
+            // shuffles give that lane its own)
             if (re_part && column && (g >= 2 || warp == 0))
-                fold[pos] = d;
+                fold[pos] = g >= 2 ? d : low_digit((unsigned)v);
             barrier();
             const int top = fold[P - 1] ? fold[P - 1] : fold[P - 2];
             bool neg = top < 0;

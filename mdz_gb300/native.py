@@ -112,6 +112,7 @@ _SIGS = {
     "mdzgpu_perturb_limbs": (C.c_int32, [C.c_int64]),
     "mdzgpu_set_wait_limit": (C.c_int, [P, C.c_int32]),
     "mdzgpu_last_escalations": (C.c_int, [P, P, C.c_int64, P, P, C.c_int64, P]),
+    "mdzgpu_last_orbit_digits": (C.c_int, [P, C.c_int32, P, C.c_int64, P, P]),
     "mdzgpu_reference_orbit_formula": (C.c_int, [P, C.c_int32, C.POINTER(MpValStruct),
                                                  C.POINTER(MpValStruct), C.c_int64, C.c_int32,
                                                  C.c_int64, P, P, P, P,
