@@ -667,12 +667,8 @@ static int perturb_steps(mdzgpu_ctx* ctx, const PerturbLaunch& p, size_t n,
     // a pixel stops at least every `budget` iterations, or when it waits for
     // the orbit: after the orbit is complete every step advances every
     // pixel, so the loop ends within depth / budget_min steps of it
-    // pixel-iterations/s of the FP32 pass: deep frames step pixels in pairs
-    const double rate = perturb_in_pairs(ctx->num_sms, p, n) ? 1.5e12 : 3.0e11;
     for (long step = 0;; ++step) {
-        const double b = rate * 8e-3 / (double)left;
-        // whole blocks of four iterations
-        const unsigned budget = (unsigned)std::min(std::max(b, 256.0), (double)(1u << 24)) & ~3u;
+        const unsigned budget = step_budget(ctx->num_sms, p, left);
         if ((rc = launch_perturb_step(ctx->num_sms, p, in, left, out, counters,
                                       (uint4*)ctx->pstate.ptr, budget, ctx->stream, ctx->ev_k0,
                                       ctx->ev_k1)))

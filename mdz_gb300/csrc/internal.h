@@ -312,8 +312,8 @@ struct PerturbLaunch {
 // pass 0: FP32 frame pass; pass 1: FP64 pass over list_in
 int launch_perturb(mdzgpu_ctx* ctx, const PerturbLaunch& p, cudaStream_t s, int pass);
 // The orbit as a cooperative producer + finisher launch that publishes its
-// progress: progress[1] digits written, [2] entries finished (in whole
-// batches of its block size), [3] producer done (final length in *o.out_len), [4] a
+// progress: progress[1] digits written, [2] entries finished (a multiple of
+// 1024 until the last: whole cache lines of every array), [3] producer done (final length in *o.out_len), [4] a
 // bounded wait gave up, [5] SM id + 1 of the producer while it runs.
 // `done` (optional) stores 1 when the launch is complete, 2 if it gave up.
 int launch_orbit_stream(const OrbitLaunch& o, int* progress, cudaStream_t s,
@@ -330,7 +330,19 @@ int launch_perturb_step(int num_sms, const PerturbLaunch& p, const unsigned* in,
                         cudaEvent_t after = nullptr);
 // Whether a step over n pixels takes two a lane (perturb_pairs_kernel): where
 // the deltas start below the FP32 range and every warp of the chip gets 64.
-bool perturb_in_pairs(int num_sms, const PerturbLaunch& p, size_t n);
+inline bool perturb_in_pairs(int num_sms, const PerturbLaunch& p, size_t n)
+{
+    return p.fractal == MDZ_MANDELBROT && p.att && p.hs_e < -160 && n >= (size_t)64 * 24 * num_sms;
+}
+// Iterations a pixel may take in a step over `left` pixels: about 8 ms of the
+// FP32 pass, in whole blocks of four.  The rate is that of the kernel that takes
+// this step: the pixels left may be fewer than the frame's.
+inline unsigned step_budget(int num_sms, const PerturbLaunch& p, unsigned left)
+{
+    const double rate = perturb_in_pairs(num_sms, p, left) ? 1.5e12 : 3.0e11;   // pixel-iterations/s
+    const double b = rate * 8e-3 / (double)left;
+    return (unsigned)(b < 256.0 ? 256.0 : b > (double)(1u << 24) ? (double)(1u << 24) : b) & ~3u;
+}
 // Orbit + FP32 pixel pass in one cooperative launch (progress words in p).
 int launch_fused(mdzgpu_ctx* ctx, const OrbitLaunch& o, const PerturbLaunch& p, cudaStream_t s);
 

@@ -3288,11 +3288,6 @@ int launch_orbit_stream(const OrbitLaunch& o, int* progress, cudaStream_t s, Don
     return MDZGPU_OK;
 }
 
-bool perturb_in_pairs(int num_sms, const PerturbLaunch& p, size_t n)
-{
-    return p.fractal == MDZ_MANDELBROT && p.att && p.hs_e < -160 && n >= (size_t)64 * 24 * num_sms;
-}
-
 int launch_perturb_step(int num_sms, const PerturbLaunch& p, const unsigned* in, unsigned n,
                         unsigned* out, unsigned* counters, uint4* state, unsigned budget,
                         cudaStream_t s, cudaEvent_t before, cudaEvent_t after)
