@@ -2503,12 +2503,14 @@ __device__ __forceinline__ void list_pixels(const PerturbLaunch& p)
             if constexpr (kDirect) {
                 const unsigned dm = __ballot_sync(0xffffffffu, done == 2);
                 if (done == 2) {
-                    // c = Z_1 + dc
+                    // c = Z_1 + dc of the orbit that starts at 0 (the Julia
+                    // family's critical one; its pixels share c)
+                    const int one = JU ? p.q0 + 1 : 1;
                     DirectPixel& q = direct[warp][nd + __popc(dm & ((1u << lane) - 1u))];
                     q.xr = fp_from(r.st.tr);
                     q.xi = fp_from(r.st.ti);
-                    q.cr = fp_from(ldexp(p.zd[1].x, p.ze[1]) + ldexp(dcm_r, p.hs_e));
-                    q.ci = fp_from(ldexp(p.zd[1].y, p.ze[1]) + ldexp(dcm_i, p.hs_e));
+                    q.cr = fp_from(ldexp(p.zd[one].x, p.ze[one]) + ldexp(dcm_r, p.hs_e));
+                    q.ci = fp_from(ldexp(p.zd[one].y, p.ze[one]) + ldexp(dcm_i, p.hs_e));
                     q.wz = r.wz;
                     q.pix = pix;
                 }
