@@ -1135,7 +1135,7 @@ __device__ __forceinline__ bool fold_certain(T zr, T zi, T Zx, T Zy, T fs, T dzm
 }
 
 // fold_certain of the FP64 pass, from the high words where they show it; hd is
-// the high word of dz's larger component (0 once the estimate is lost).
+// the high word of dz's larger component.
 template <int FR>
 __device__ __forceinline__ bool fold_certain_bits(double zr, double zi, double Zx, double Zy,
                                                   double fs, int hd)
@@ -1209,23 +1209,22 @@ __device__ __forceinline__ bool fold_err_hopeless(const PixState<double>& st)
 
 // Within reach of the bailout: |z|^2 > 4 - 2^-14, or nearer to 4 than 2^9
 // times the error estimate of z.
-__device__ __forceinline__ bool near_bailout(float mag, const PixState<float>& st, bool lost_track)
+__device__ __forceinline__ bool near_bailout(float mag, const PixState<float>& st)
 {
     const float dv = mag - 4.f;
-    return dv > -6.1035156e-5f || (!lost_track && dv * dv <= st.kb * st.e2);
+    return dv > -6.1035156e-5f || dv * dv <= st.kb * st.e2;
 }
 
-__device__ __forceinline__ bool near_bailout(double mag, const PixState<double>& st,
-                                             bool lost_track)
+__device__ __forceinline__ bool near_bailout(double mag, const PixState<double>& st)
 {
     // |z|^2 < 3.875 and kb e2 < 2^-14.8 < 0.125^2
     if ((unsigned)hi_of(mag) < 0x400f0000u
-        && (lost_track || log_sum(st.kb, st.e2) < 0x3ff00000u + 0x3f000000u))
+        && log_sum(st.kb, st.e2) < 0x3ff00000u + 0x3f000000u)
         return false;
     bool r;
     do {
         const double dv = add_here(mag, -4.0);
-        r = dv > -6.1035156e-5 || (!lost_track && mul_here(dv, dv) <= mul_here(st.kb, st.e2));
+        r = dv > -6.1035156e-5 || mul_here(dv, dv) <= mul_here(st.kb, st.e2);
     } while (once());
     return r;
 }
@@ -1271,26 +1270,27 @@ __device__ __forceinline__ bool needs_rescale(T tr, T ti, int& k)
 }
 
 // The every-4th-iteration check.  A trajectory whose estimate passed the
-// limits goes to the next pass, except in the FP64 pass of a folded
-// formula: there it is marked `lost_track` and its later decisions are no
-// longer sent to the multi-limb pass, since an error that large means the
-// pixel's orbit is chaotic beyond what any fixed precision resolves (MPFR
-// at the reference's precision and at twice it disagree there); such a
-// pixel keeps its FP64 count, as the reference keeps its own.  (The
-// Mandelbrot map is conformal: there a large estimate comes from rebases,
-// and the multi-limb pass settles the pixel.)  Returns true when the pixel
-// stops here, flagged.
+// limits goes to the next pass, except in the FP64 pass of a folded formula:
+// there it is iterated directly from here (fold_direct) and not sent to the
+// multi-limb pass, since an error that large means the pixel's orbit is chaotic
+// beyond what any fixed precision resolves (MPFR at the reference's precision
+// and at twice it disagree there); such a pixel keeps that count, as the
+// reference keeps its own.  (The Mandelbrot map is conformal: there a large
+// estimate comes from rebases, and the multi-limb pass settles the pixel.)
+enum Checkpoint { kGoOn, kNextPass, kDirect };
+
 template <class T, int FR>
-__device__ __forceinline__ bool fold_checkpoint(const PerturbLaunch& p, const PixState<T>& st,
-                                                float& lost, bool& lost_track)
+__device__ __forceinline__ Checkpoint fold_checkpoint(const PerturbLaunch& p,
+                                                      const PixState<T>& st, float& lost)
 {
+    bool direct = false;
     if (fold_err_hopeless(st)) {
         if (sizeof(T) == 4 || FR == MDZ_MANDELBROT)
             lost = fmaxf(lost, 64.f);
         else
-            lost_track = true;
+            direct = true;
     }
-    return lost > p.lost_limit && p.flag_out != nullptr;
+    return lost > p.lost_limit && p.flag_out != nullptr ? kNextPass : direct ? kDirect : kGoOn;
 }
 
 // After a rebase (t, e replaced by Z_m + dz in FP64): the error carries
@@ -1767,7 +1767,6 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
     // pass counts the bits its rebases cancel instead.
     constexpr bool kTrack = FR != MDZ_MANDELBROT || sizeof(T) == 8;
     const T grow = (T)4;
-    bool lost_track = false;   // FP64: the estimate passed its limits
     float lost_sink = 0.f;
     float& rebase_lost = kTrack ? lost_sink : r.lost;
     if (kTrack)
@@ -1835,7 +1834,7 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
                     zr = Mant<T>::fma_(st.s, st.tr, Zx);
                     zi = Mant<T>::fma_(st.s, st.ti, Zy);
                 }
-                if (fold_checkpoint<T, FR>(p, st, r.lost, lost_track)) {
+                if (fold_checkpoint<T, FR>(p, st, r.lost) == kNextPass) {
                     r.mag = (float)magT;
                     count = 0;
                     return 1;  // the next pass redoes the pixel
@@ -2041,28 +2040,22 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
             if (FR != MDZ_MANDELBROT && (!kVar || (wz & 1u))) {
                 // with dz below the T range (s = 0) a fold is out of reach
                 // unless the entry is marked: the same choice as the blocks
-                // (a lost estimate leaves only the rounding margin: the side
-                // is still decided exactly, its error no longer matters)
                 bool fast = !careful && !axis_bit(p, m);
                 if constexpr (sizeof(T) == 8) {
-                    const int hd = lost_track ? 0
-                                              : max(hi_of(st.tr) & 0x7fffffff,
-                                                    hi_of(st.ti) & 0x7fffffff)
-                                                    + st.e * (1 << 20);
+                    const int hd = max(hi_of(st.tr) & 0x7fffffff, hi_of(st.ti) & 0x7fffffff)
+                                   + st.e * (1 << 20);
                     if (fast && !(st.s == (T)0)
                         && !fold_certain_bits<FR>(zr, zi, Zx, Zy, fs, hd)) {
                         do {
                             const T dzm = mul_here(st.sm, fmax(fabs(st.tr), fabs(st.ti)));
-                            fast = fold_certain<T, FR>(zr, zi, Zx, Zy, fs,
-                                                       lost_track ? (T)0 : dzm);
+                            fast = fold_certain<T, FR>(zr, zi, Zx, Zy, fs, dzm);
                         } while (once());
                     }
                 } else {
                     fast = fast
                            && (st.s == (T)0
-                               || fold_certain<T, FR>(
-                                   zr, zi, Zx, Zy, fs,
-                                   lost_track ? (T)0 : st.sm * fmax(fabs(st.tr), fabs(st.ti))));
+                               || fold_certain<T, FR>(zr, zi, Zx, Zy, fs,
+                                                      st.sm * fmax(fabs(st.tr), fabs(st.ti))));
                 }
                 if (fast) {
                     fold_fast_step<T, FR>(st, Zx, Zy, fs);
@@ -2070,8 +2063,7 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
                     const int e0 = st.e;
                     float unsure = 0.f;
                     fold_step<T, FR>(p, m, st, dcf_r, dcf_i, dcm_r, dcm_i, dce, unsure);
-                    if (!lost_track)
-                        r.lost += unsure;
+                    r.lost += unsure;
                     if (st.e != e0)
                         st.e2 = Mant<T>::scale(st.e2, 2 * (e0 - st.e));
                 }
@@ -2101,11 +2093,11 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
         }
         if (kTrack) {
             // the band widens to 2^9 err where the error estimate of z is
-            // larger (not once the estimate is lost: its decisions stand)
-            if (near_bailout(magT, st, lost_track)) {
+            // larger
+            if (near_bailout(magT, st)) {
                 bool unsure;
                 const bool esc = escape_fold<T>(p, m, st, unsure);
-                if (unsure && !lost_track)
+                if (unsure)
                     r.lost = fmaxf(r.lost, 64.f);
                 if (esc) {
                     r.mag = (float)magT;
@@ -2178,12 +2170,13 @@ __device__ int perturb_run(const PerturbLaunch& p, PixRun<T>& r, double dcm_r, d
                 zr = Mant<T>::fma_(st.s, st.tr, Zx);
                 zi = Mant<T>::fma_(st.s, st.ti, Zy);
             }
-            if (kTrack && fold_checkpoint<T, FR>(p, st, r.lost, lost_track)) {
+            const Checkpoint next = kTrack ? fold_checkpoint<T, FR>(p, st, r.lost) : kGoOn;
+            if (next == kNextPass) {
                 r.mag = (float)magT;
                 count = 0;
                 return 1;  // the next pass redoes the pixel
             }
-            if (FR != MDZ_MANDELBROT && sizeof(T) == 8 && lost_track) {
+            if (FR != MDZ_MANDELBROT && sizeof(T) == 8 && next == kDirect) {
                 // the caller iterates the rest directly, from z after wz
                 st.tr = zr;
                 st.ti = zi;
