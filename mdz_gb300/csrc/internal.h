@@ -176,13 +176,23 @@ constexpr int split_list_per_sm()
     return N >= 16 ? 64 : N >= 10 ? 32 : 0;
 }
 // Of these, lists of at most this many pixels an SM go to mp_pixel_kernel: a
-// block's iteration takes 1.25 us at N = 34, and each further pixel an SM adds
-// 0.06 (16000 iterations, 2.8 pixels an SM: 20.1 ms, 35.6 in mp_split_kernel;
-// 8.5: 25.9 and 36.4); at N = 16 0.9 and 0.06 (2.6 pixels an SM: 9.7 and 9.2).
+// block's iteration takes 0.9 us at N = 24 and 34 and each further pixel an SM
+// adds 0.06, with a jump where a ninth pixel waits for a second round of blocks.
+// Lists to depth 10600, ms in mp_pixel_kernel and in mp_split_kernel:
+//   N = 16: 0.3 pixels an SM 9.2 and 8.0, 2.8 11.5 and 9.3
+//   N = 20: 0.7 10.0 and 10.2, 2.7 10.9 and 11.9, 5.4 12.7 and 12.0
+//   N = 24: 0.7 10.0 and 12.3, 2.9 11.2 and 14.8, 5.1 12.5 and 15.0, 11.5 18.9
+//           and 15.1
+//   N = 28: 3.0 12.7 and 17.8, 6.1 14.8 and 17.8, 7.8 17.8 and 17.8, 9.6 19.0 and
+//           17.9
+//   N = 34: 3.0 12.5 and 24.0, 7.7 18.1 and 23.6, 9.2 26.3 and 23.7, 15.0 34.3 and
+//           23.7
+//   N = 36: 4.9 17.2 and 33.5, 9.0 27.8 and 33.6, 12.9 33.9 and 33.6, 16.5 43.5 and
+//           33.6
 template <int N>
 constexpr int pixel_list_per_sm()
 {
-    return N >= 34 ? 16 : N >= 28 ? 6 : N >= 24 ? 3 : 0;
+    return N >= 36 ? 12 : N >= 34 ? 8 : N >= 28 ? 6 : N >= 24 ? 3 : 0;
 }
 int launch_mp(mdzgpu_ctx* ctx, const MpLaunch& p, cudaStream_t s);
 // Kernels launch_mp launches for a list's first chunk.

@@ -146,9 +146,12 @@ __host__ __device__ constexpr int block_threads()
 
 // A frame launch takes one block an SM, whose warps merge as pixels finish
 // (pixel_feed.cuh): 320x240 at 80 bits, counts 0.70 of the depth on average,
-// 8.08 ms in four blocks of four warps an SM, 6.8 in one of 16.  At most 16
-// warps (with 24 nothing gains, with 8 the multiplier waits: 640x480-class
-// frames at 4 and 10 words).
+// 8.08 ms in four blocks of four warps an SM, 6.8 in one of 16.  16 warps hide the
+// multiplier's latency best as long as the registers go round, up to 16 words
+// (128 a thread, a few spilled): 640x480 to depth 500, all pixels to the end, in
+// 16, 12 and 8 warps 4.27, 4.68, 4.74 ms at 10 words, 5.40, 6.02, 5.89 at 12, 7.88,
+// 8.81, 8.35 at 16.  At 20 words 12 warps (11.4 ms, 11.5 with 8), above 8: 24 words
+// 15.6 ms and 14.7 in 12, but 320x240 to depth 1000 7.85 and 8.93.
 template <int N>
 __host__ __device__ constexpr int frame_block()
 {

@@ -27,7 +27,7 @@ JULIA = json.loads((GOLD / "perturb_julia_views.json").read_text())
 
 # pixels an SM, by words (split_list_per_sm, pixel_list_per_sm)
 SPLIT = {10: 32, 12: 32, 16: 64, 20: 64, 24: 64, 28: 64, 34: 64, 36: 64}
-PIXEL = {24: 3, 28: 6, 34: 16, 36: 16}
+PIXEL = {24: 3, 28: 6, 34: 8, 36: 12}
 
 # kernel, view, log2 width, precision, words, W, H, depth
 CASES = [
