@@ -51,14 +51,14 @@ VIEWS = json.loads((ROOT / "tests" / "golden" / "views.json").read_text())
 # (8 flops); the roofline counts the algorithmic 16 against the FP32 flop
 # peak (2 flops per FFMA lane).
 ALGO_OPS_PER_PIXEL_ITER = 16
-# DRAM bytes (read + written) of one pixel-step launch of the 1920x1080
-# 2^-1000 frame: ncu dram__bytes_read.sum + dram__bytes_write.sum (one pass,
-# --clock-control none) over launches 61-63 of one frame, 74.7 MB read and
-# 11.6-14.6 MB written each, taken with one pixel a lane
-# (profiles/perturb_step_kernel_c4_traffic.md); two a lane move the same state.
+# DRAM bytes (read + written) of one pixel-step launch (perturb_pairs_kernel)
+# of the 1920x1080 2^-1000 frame: ncu dram__bytes_read.sum +
+# dram__bytes_write.sum (one pass, --clock-control none) over launches 21-23 of
+# one frame, 75.5 MB read and 13.9-17.0 MB written each
+# (profiles/perturb_step_kernel_c4_traffic.md).
 # The pixel state (32 B per unfinished pixel) goes in and out once a launch;
 # the reference orbit (3.2 MB of float4 entries) is read from L2.
-STEP_LAUNCH_DRAM_BYTES = 87.6e6
+STEP_LAUNCH_DRAM_BYTES = 90.6e6
 # rows of the frame rendered by the plain multi-limb kernel: 1920 x 64 pixels
 # = 3840 warps of 8x4-pixel tiles, about three full waves of the resident
 # warps at 34 words (240 registers: 8 warps per SM x 152 SMs)

@@ -24,10 +24,10 @@
 //    tiles are added as three distributed numbers (lane carries as above); the
 //    result is the window F .. F + 64 NL of that sum.
 //
-// What bounds it is the integer multiplier, 1.1 SM cycles a warp for each
-// 32x32-bit product, and the lanes that wait for the group's longest tile
-// (tiles hold 1 to NL / 2 pairs; three rounds of G tiles at NL = 40 keep 75% of
-// the lanes at work).  64-bit products (mad.lo/hi.u64: a dozen instructions for
+// What bounds it is latency with few warps: 96x64 pixels are 15% of an SM's, at
+// 44% issue (multiplier 33%, ALU 33%).  A product costs an addition of its carry
+// as well, and lanes wait for the group's longest tile (tiles hold 1 to NL / 2
+// pairs; three rounds of G tiles at NL = 40 keep 75% of the lanes at work).  64-bit products (mad.lo/hi.u64: a dozen instructions for
 // four 32-bit products, a load each) took 45.8 ms for a 96x64 view at 2176 bits,
 // this form 27.2 ms.
 //

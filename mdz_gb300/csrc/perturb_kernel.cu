@@ -3042,8 +3042,8 @@ __device__ __forceinline__ bool deep_pairs(const PerturbLaunch& p, PairStage& st
 // perturb_step_kernel for a Mandelbrot frame whose deltas start below the FP32
 // range: a lane takes two pixels and steps them together as long as they are
 // at the same orbit entry (from the frame's start until one of them leaves
-// the deep part or rebases).  What bounds it is issue: 9.5 warp instructions a
-// pixel-iteration one pixel at a time.
+// the deep part or rebases).  What bounds it is the latency of a step's two
+// dependent packed FMAs with one pair a lane (issue 54%, FMA pipe 51%).
 template <bool WANT_MAG>
 __global__ void __launch_bounds__(256, 3) perturb_pairs_kernel(PerturbLaunch p, FrameStep q)
 {
