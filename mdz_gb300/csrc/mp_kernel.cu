@@ -58,6 +58,18 @@ __device__ __forceinline__ float fx_top_float(const uint32_t (&x)[N])
            + (float)x[N - 2] * 1.3877788e-17f /* 2^-56 */;
 }
 
+// Whether a pixel's |z|^2 is formed when it is done, from the squares' top words
+// (four registers), and not in the step that ends it: the step then has no
+// branch for it.  3000 iterations of one pixel at 4 words 0.73 ms and 0.80 (the
+// kernel before MpOrbit 0.71), 80 and 256 bits, 320x240, 6.9 and 18.0 ms and 7.2 and
+// 18.9; from 16 to 34 words 3% to 1%.  At 36 words the registers do not go round:
+// 1088 bits 67.7 ms and 64.9.
+template <int N>
+constexpr bool late_mag()
+{
+    return N <= 34;
+}
+
 // A pixel's orbit between iterations: |wre|, |wim| with their sign masks and
 // wre^2 - wim^2, after `wz` iterations.
 template <int N>
@@ -65,10 +77,11 @@ struct MpOrbit {
     uint32_t wre[N], wim[N], d[N];
     uint32_t sre, sim;
     uint32_t wz;
+    uint32_t top[late_mag<N>() ? 4 : 1];   // of wim^2 and of wre^2, high word first
 };
 
-// The squares of |wre|, |wim|: sets d; returns whether |z|^2 > 4, and |z|^2
-// (rounded) when it is or when `want_mag`.
+// The squares of |wre|, |wim|: sets d (and top); returns whether |z|^2 > 4, and
+// else |z|^2 (rounded) when it is or when `want_mag`.
 template <int N>
 __device__ __forceinline__ bool mp_squares(MpOrbit<N>& o, bool want_mag, float& mag)
 {
@@ -78,8 +91,14 @@ __device__ __forceinline__ bool mp_squares(MpOrbit<N>& o, bool want_mag, float& 
     fx::sqr_trunc<N>(o.wre, acc);
     fx::extract<N, 24>(acc, wre2);
     const bool escaped = fx::sum_gt4<N>(wim2, wre2);
-    if (escaped || want_mag)
+    if constexpr (late_mag<N>()) {
+        o.top[0] = wim2[N - 1];
+        o.top[1] = wim2[N - 2];
+        o.top[2] = wre2[N - 1];
+        o.top[3] = wre2[N - 2];
+    } else if (escaped || want_mag) {
         mag = fx_top_float<N>(wim2) + fx_top_float<N>(wre2);
+    }
     fx::sub<N>(wre2, wim2, o.d);
     return escaped;
 }
@@ -93,6 +112,14 @@ __device__ __forceinline__ void mp_start(MpOrbit<N>& o)
     o.sim = fx::abs_inplace<N>(o.wim);
     o.wz = 0;
     mp_squares<N>(o, false, mag);   // z_0 = c is not tested
+}
+
+// |z|^2 of a z whose square the format may not hold (signed wre, wim).
+template <int N>
+__device__ __forceinline__ float mp_far_mag(const MpOrbit<N>& o)
+{
+    const float a = fx_top_float<N>(o.wre), b = fx_top_float<N>(o.wim);
+    return a * a + b * b;
 }
 
 // The next iteration.  Returns true when z escaped; mag as mp_squares.
@@ -114,13 +141,26 @@ __device__ __forceinline__ bool mp_step(MpOrbit<N>& o, const CG& c_re, const CG&
                             : 0u;
     fx::add_signed<N>(c_re, o.d, md, o.wre);
     if (fx::big<N>(o.wre) || fx::big<N>(o.wim)) {
-        const float a = fx_top_float<N>(o.wre), b = fx_top_float<N>(o.wim);
-        mag = a * a + b * b;
+        if constexpr (!late_mag<N>())
+            mag = mp_far_mag<N>(o);
         return true;
     }
     o.sre = fx::abs_inplace<N>(o.wre);
     o.sim = fx::abs_inplace<N>(o.wim);
     return mp_squares<N>(o, want_mag, mag);
+}
+
+// |z|^2 of a finished pixel; mag as its last step left it.
+template <int N>
+__device__ __forceinline__ float mp_mag(const MpOrbit<N>& o, float mag)
+{
+    if constexpr (late_mag<N>()) {
+        if (fx::big<N>(o.wre) || fx::big<N>(o.wim))
+            return mp_far_mag<N>(o);
+        const uint32_t im[2] = {o.top[1], o.top[0]}, re[2] = {o.top[3], o.top[2]};
+        return fx_top_float<2>(im) + fx_top_float<2>(re);
+    }
+    return mag;
 }
 
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
@@ -151,7 +191,8 @@ __host__ __device__ constexpr int block_threads()
 // (128 a thread, a few spilled): 640x480 to depth 500, all pixels to the end, in
 // 16, 12 and 8 warps 4.27, 4.68, 4.74 ms at 10 words, 5.40, 6.02, 5.89 at 12, 7.88,
 // 8.81, 8.35 at 16.  At 20 words 12 warps (11.4 ms, 11.5 with 8), above 8: 24 words
-// 15.6 ms and 14.7 in 12, but 320x240 to depth 1000 7.85 and 8.93.
+// 15.6 ms and 14.7 in 12, but 320x240 to depth 1000 7.85 and 8.93.  (Taken with
+// |z|^2 formed in the step; see late_mag.)
 template <int N>
 __host__ __device__ constexpr int frame_block()
 {
@@ -298,7 +339,7 @@ __global__ void __launch_bounds__(frame_block<N>(), 1) mp_frame_kernel(MpLaunch 
                     const size_t at = (size_t)lrow * p.W + ix;
                     p.out[at] = (int32_t)n;
                     if (p.mag)
-                        p.mag[at] = mag;
+                        p.mag[at] = mp_mag<N>(o, mag);
                     its += n ? n : p.depth;
                     active = false;
                     band = lrow / kTileH;
@@ -821,7 +862,7 @@ __global__ void __launch_bounds__(block_threads<N>()) serve_mp_kernel(ServeDev* 
                 if (escaped || o.wz >= depth) {
                     rq.pl.out[pix] = escaped ? (int32_t)o.wz : 0;
                     if (rq.pl.mag)
-                        rq.pl.mag[pix] = mag;
+                        rq.pl.mag[pix] = mp_mag<N>(o, mag);
                     done = true;
                 } else {
 #pragma unroll
